@@ -22,6 +22,10 @@ struct Ctx
     // or Rectangular<1> (rect = 0: the plaquette staple)
     int rect = 0;
     double cp = 1.0, cr = 0.0;
+    // two-link products (a gauge field) and their outer staples (a full field) for the rectangle
+    // forces over all links; null: no memory for them, the rectangles are multiplied out directly
+    void* rectD = nullptr;
+    void* rectE = nullptr;
     unsigned* order = nullptr;    // the handle's launch counter for alternating site orders
 };
 

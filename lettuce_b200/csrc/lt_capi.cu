@@ -52,6 +52,19 @@ int ensure(lt_lattice* h, void** p, size_t bytes)
     return LT_OK;
 }
 
+// The scratch fields of a rectangle force over all links.  On the largest lattices there may be no
+// memory for them; the force is then multiplied out path by path, as it is without them.
+void ensure_rect(lt_lattice* h)
+{
+    if (h->rectE) return;
+    if (cudaMalloc(&h->rectD, h->be->gauge_bytes(h->g)) == cudaSuccess &&
+        cudaMalloc(&h->rectE, h->be->full_bytes(h->g)) == cudaSuccess)
+        return;
+    (void)cudaGetLastError();
+    if (h->rectD) cudaFree(h->rectD);
+    h->rectD = h->rectE = nullptr;
+}
+
 int ensure_aos(lt_lattice* h) { return ensure(h, (void**)&h->d_aos, (size_t)4 * h->g.V * 18 * sizeof(double)); }
 
 // Kernel-launch status after a batch of launches
@@ -111,6 +124,7 @@ int flow_steps(lt_lattice* h, double eps, int n_step, int integrator = LT_FLOW_R
     if (ns > 1) LT_TRY(ensure(h, &h->Z, h->be->alg_bytes(h->g)));
     const bool zeuthen = h->flow_action == LT_FLOW_ACTION_ZEUTHEN;
     if (zeuthen || h->be->flow_split()) LT_TRY(ensure(h, &h->Xz, h->be->alg_bytes(h->g)));
+    if (zeuthen || h->act_radius == 2) ensure_rect(h);
     const lt::Ctx c = h->ctx();
     for (int k = 0; k < n_step; ++k)
         for (int j = 0; j < ns; ++j)
@@ -278,6 +292,7 @@ int kick(lt_lattice* h, double beta, double eps, const MetaDParams* md, bool sub
         LT_TRY(metad_force_now(h, md, submeasure));
         F = h->F;
     }
+    if (h->act_radius == 2) ensure_rect(h);
     h->be->momenta(h->ctx(), h->U, h->P, F, beta / 6.0, eps);
     return launched("momenta");
 }
@@ -839,7 +854,7 @@ int lt_destroy(lt_lattice* h)
     if (h->stream) cudaStreamSynchronize(h->stream);
     void* bufs[] = { h->U,   h->U2,   h->Z,        h->P,       h->F,     h->Ubak,   h->R,      h->chainA,
                      h->Lam, h->Tloc, h->partials, h->results, h->d_aos, h->status, h->chainB, h->Xz,
-                     h->tensor };
+                     h->tensor, h->rectD, h->rectE };
     for (void* p : bufs)
         if (p) cudaFree(p);
     for (void* p : h->levels) cudaFree(p);
@@ -1554,6 +1569,7 @@ int lt_gauge_force(lt_lattice* h, double beta, double* force_out)
     if (!force_out) return lt::set_error(LT_ERR_ARG, "lt_gauge_force: null pointer");
     LT_TRY(ensure(h, &h->F, h->be->alg_bytes(h->g)));
     LT_CK(cudaMemsetAsync(h->F, 0, h->be->alg_bytes(h->g), h->stream));
+    if (h->act_radius == 2) ensure_rect(h);
     h->be->momenta(h->ctx(), h->U, h->F, nullptr, beta / 6.0, 1.0);
     LT_TRY(ensure_aos(h));
     h->be->alg_to_aos(h->ctx(), h->F, h->d_aos);

@@ -81,6 +81,8 @@ struct lt_lattice
     // force of the gradient flow run into this handle (lt_set_flow_action): the gauge action's
     // (LT_FLOW_ACTION_GAUGE, the reference's GradientFlowKernel) or the Zeuthen flow's
     int flow_action = LT_FLOW_ACTION_GAUGE;
+    void* rectD = nullptr;       // two-link products of the rectangle forces (link field)
+    void* rectE = nullptr;       // and their outer staples (full matrices)
     void* Xz = nullptr;          // Luescher-Weisz force of a Zeuthen flow stage (algebra)
     double* tensor = nullptr;    // FullTensor4D of lt_clover_tensor (FP64, reference layout)
     mutable unsigned order = 0;  // launches of the order-alternating sweep and flow kernels
@@ -96,6 +98,8 @@ struct lt_lattice
         c.rect = act_radius == 2;
         c.cp = act_cp;
         c.cr = act_cr;
+        c.rectD = rectD;
+        c.rectE = rectE;
         c.order = &order;
         return c;
     }

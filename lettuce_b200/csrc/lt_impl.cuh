@@ -73,6 +73,26 @@ template <typename T, int NR> class BackendImpl final : public Backend
     static Clov<T> clov(const void* p, const Geom& g) { Clov<T> a; a.p = (T*)p; a.vh = g.vh; return a; }
     static Full<double> full64(const void* p, const Geom& g) { Full<double> a; a.p = (cx<double>*)p; a.vh = g.vh; return a; }
 
+    static RectFields<T, NR> rect_fields(const Ctx& c) { return { gauge(c.rectD, c.g), full(c.rectE, c.g) }; }
+
+    // D and E of all links of U (lt_kernels.cuh) for a rectangle force that follows on the stream
+    static void prepare_rect(const Ctx& c, const void* U, double cr)
+    {
+        const int nb = nblocks(c.g.V, kSitesPerBlock);
+        launch_chained(k_two_links<T, NR>, nb, 4 * kSitesPerBlock, c.stream, gauge(U, c.g), gauge(c.rectD, c.g), c.g,
+                       next_order(c));
+        if constexpr (kStaged)
+        {
+            prefer_shared<k_rect_outer_staged<0>>();
+            launch_chained(k_rect_outer_staged<0>, nb, 4 * kSitesPerBlock, c.stream, gauge(U, c.g), rect_fields(c), c.g,
+                           (T)cr, next_order(c));
+        }
+        else
+            launch_chained(k_rect_outer<T, NR>, nb, 4 * kSitesPerBlock, c.stream, gauge(U, c.g), rect_fields(c), c.g,
+                           (T)cr, next_order(c));
+    }
+    static Act act(const Ctx& c, bool rect) { return !rect ? Act::Wilson : c.rectE ? Act::TwoLink : Act::Direct; }
+
     static void finish(const Ctx& c, int slot, int nslot)
     {
         k_reduce_final<<<nslot, kRedThreads, 0, c.stream>>>(c.partials + (size_t)slot * kRedBlocks, kRedBlocks,
@@ -232,35 +252,62 @@ public:
             if (X)
             {
                 const int nb = nblocks(c.g.V, kSitesPerBlock);
-                launch_chained(c.rect ? k_flow_force<T, NR, true> : k_flow_force<T, NR, false>, nb, 4 * kSitesPerBlock,
-                               c.stream, gauge(Uin, c.g), alg(X, c.g), c.g, (T)c.cp, (T)c.cr, next_order(c));
+                force(c, Uin, X, c.rect, c.cp, c.cr);
                 launch_chained(k_flow_update<T, NR>, nb, 4 * kSitesPerBlock, c.stream, gauge(Uin, c.g),
                                gauge(Uout, c.g), alg(Z, c.g), alg(X, c.g), c.g, (T)c_old, (T)c_new, (T)c_exp, read_z,
                                write_z, next_order(c));
                 return;
             }
         }
+        const int nb = nblocks(c.g.V, kSitesPerBlock);
+        const Act a = act(c, c.rect);
+        if (a == Act::TwoLink) prepare_rect(c, Uin, c.cr);
         if constexpr (kStaged)
         {
-            if (!c.rect)
+            if (a != Act::Direct)
             {
-                prefer_shared<k_flow_stage_staged<0>>();
-                launch_chained(k_flow_stage_staged<0>, nblocks(c.g.V, kSitesPerBlock), 4 * kSitesPerBlock, c.stream,
-                               gauge(Uin, c.g), gauge(Uout, c.g), alg(Z, c.g), c.g, (T)c_old, (T)c_new, (T)c_exp,
-                               read_z, write_z, next_order(c));
+                prefer_shared<k_flow_stage_staged<Act::Wilson>>();
+                prefer_shared<k_flow_stage_staged<Act::TwoLink>>();
+                launch_chained(a == Act::Wilson ? k_flow_stage_staged<Act::Wilson> : k_flow_stage_staged<Act::TwoLink>,
+                               nb, 4 * kSitesPerBlock, c.stream, gauge(Uin, c.g), gauge(Uout, c.g), alg(Z, c.g), c.g,
+                               (T)c_old, (T)c_new, (T)c_exp, read_z, write_z, rect_fields(c), (T)c.cp, (T)c.cr,
+                               next_order(c));
                 return;
             }
         }
-        launch_chained(c.rect ? k_flow_stage<T, NR, true> : k_flow_stage<T, NR, false>, nblocks(c.g.V, kSitesPerBlock),
-                       4 * kSitesPerBlock, c.stream, gauge(Uin, c.g), gauge(Uout, c.g), alg(Z, c.g), c.g, (T)c_old,
-                       (T)c_new, (T)c_exp, read_z, write_z, (T)c.cp, (T)c.cr, next_order(c));
+        launch_chained(a == Act::Wilson    ? k_flow_stage<T, NR, Act::Wilson>
+                       : a == Act::TwoLink ? k_flow_stage<T, NR, Act::TwoLink>
+                                           : k_flow_stage<T, NR, Act::Direct>,
+                       nb, 4 * kSitesPerBlock, c.stream, gauge(Uin, c.g), gauge(Uout, c.g), alg(Z, c.g), c.g, (T)c_old,
+                       (T)c_new, (T)c_exp, read_z, write_z, rect_fields(c), (T)c.cp, (T)c.cr, next_order(c));
+    }
+    // X <- Algebra(st U^dag) of every link
+    static void force(const Ctx& c, const void* U, void* X, bool rect, double cp, double cr)
+    {
+        const int nb = nblocks(c.g.V, kSitesPerBlock);
+        const Act a = act(c, rect);
+        if (a == Act::TwoLink) prepare_rect(c, U, cr);
+        if constexpr (kStaged)
+        {
+            if (a == Act::TwoLink)
+            {
+                prefer_shared<k_flow_force_staged<0>>();
+                launch_chained(k_flow_force_staged<0>, nb, 4 * kSitesPerBlock, c.stream, gauge(U, c.g), alg(X, c.g),
+                               c.g, rect_fields(c), (T)cp, (T)cr, next_order(c));
+                return;
+            }
+        }
+        launch_chained(a == Act::Wilson    ? k_flow_force<T, NR, Act::Wilson>
+                       : a == Act::TwoLink ? k_flow_force<T, NR, Act::TwoLink>
+                                           : k_flow_force<T, NR, Act::Direct>,
+                       nb, 4 * kSitesPerBlock, c.stream, gauge(U, c.g), alg(X, c.g), c.g, rect_fields(c), (T)cp, (T)cr,
+                       next_order(c));
     }
     void flow_zeuthen_stage(const Ctx& c, const void* Uin, void* Uout, void* Z, void* X, double c_old, double c_new,
                             double c_exp, int read_z, int write_z, double cp, double cr) const override
     {
         const int nb = nblocks(c.g.V, kSitesPerBlock);
-        launch_chained(k_flow_force<T, NR, true>, nb, 4 * kSitesPerBlock, c.stream, gauge(Uin, c.g), alg(X, c.g),
-                       c.g, (T)cp, (T)cr, next_order(c));
+        force(c, Uin, X, true, cp, cr);
         launch_chained(k_flow_zeuthen_stage<T, NR>, nb, 4 * kSitesPerBlock, c.stream, gauge(Uin, c.g),
                        gauge(Uout, c.g), alg(Z, c.g), alg(X, c.g), c.g, (T)c_old, (T)c_new, (T)c_exp, read_z,
                        write_z, next_order(c));
@@ -280,19 +327,26 @@ public:
 
     void momenta(const Ctx& c, const void* U, void* P, const void* F, double coef, double eps) const override
     {
+        const int nb = nblocks(c.g.V, kSitesPerBlock);
+        const Act a = act(c, c.rect);
+        if (a == Act::TwoLink) prepare_rect(c, U, c.cr);
         if constexpr (kStaged)
         {
-            if (!c.rect)
+            if (a != Act::Direct)
             {
-                prefer_shared<k_momenta_staged<0>>();
-                k_momenta_staged<0><<<nblocks(c.g.V, kSitesPerBlock), 4 * kSitesPerBlock, 0, c.stream>>>(
-                    gauge(U, c.g), alg(P, c.g), alg(F, c.g), c.g, (T)coef, (T)eps, F != nullptr);
+                prefer_shared<k_momenta_staged<Act::Wilson>>();
+                prefer_shared<k_momenta_staged<Act::TwoLink>>();
+                auto k = a == Act::Wilson ? k_momenta_staged<Act::Wilson> : k_momenta_staged<Act::TwoLink>;
+                k<<<nb, 4 * kSitesPerBlock, 0, c.stream>>>(gauge(U, c.g), alg(P, c.g), alg(F, c.g), c.g, (T)coef, (T)eps,
+                                                           F != nullptr, rect_fields(c), (T)c.cp, (T)c.cr);
                 return;
             }
         }
-        auto k = c.rect ? k_momenta<T, NR, true> : k_momenta<T, NR, false>;
-        k<<<nblocks(c.g.V, kSitesPerBlock), 4 * kSitesPerBlock, 0, c.stream>>>(
-            gauge(U, c.g), alg(P, c.g), alg(F, c.g), c.g, (T)coef, (T)eps, F != nullptr, (T)c.cp, (T)c.cr);
+        auto k = a == Act::Wilson    ? k_momenta<T, NR, Act::Wilson>
+                 : a == Act::TwoLink ? k_momenta<T, NR, Act::TwoLink>
+                                     : k_momenta<T, NR, Act::Direct>;
+        k<<<nb, 4 * kSitesPerBlock, 0, c.stream>>>(gauge(U, c.g), alg(P, c.g), alg(F, c.g), c.g, (T)coef, (T)eps,
+                                                   F != nullptr, rect_fields(c), (T)c.cp, (T)c.cr);
     }
     void fields(const Ctx& c, void* U, const void* P, double eps) const override
     {

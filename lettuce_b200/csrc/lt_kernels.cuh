@@ -763,6 +763,214 @@ LT_D M3<T> staple_rect(const Gauge<T, NR>& U, const Geom& g, int par, int i, con
     return st;
 }
 
+// The same sum from fields computed once for all links (k_two_links, k_rect_outer), for the
+// kernels that need the staples of every link of one gauge field (flow stages, forces):
+//   D_mu(x) = U_mu(x) U_mu(x+mu), one link of length two, and
+//   E_mu(x) = c_rect sum_{nu, +-} U_nu(x) D_mu(x+nu) U_nu(x+2mu)^dag, its plaquette-like staple.
+// The loops orthogonal to the link are then plaquette paths with D_nu in place of U_nu, and the
+// loops along it are E_mu(x) U_mu(x+mu)^dag + U_mu(x-mu)^dag E_mu(x-mu): 39 products a link for
+// c_plaq StaplePlaq + c_rect StapleRect (1 for D, 12 for E, 26 here) against 78 multiplied out link
+// by link, and 54 link loads against 102.  Bound by instruction issue like the plain staple.  A
+// Zeuthen RK3 step at 48 x 24^3 on two-row FP32 links with its measurements took 8.8 ms path by path
+// and takes 3.4 ms; the dynamics of four OMF_4 steps with the Luescher-Weisz action at 24 x 20^3 on
+// FP32 links 14.8 and 6.6 ms.
+template <typename T, int NR> struct RectFields
+{
+    Gauge<T, NR> D;
+    Full<T> E;
+};
+
+// a += coef sum over nu != mu of the six paths
+//   A_nu(x) B_mu(x + SN nu) A_nu(x + SM mu)^dag + A_nu(x - SN nu)^dag B_mu(x - SN nu) A_nu(x - SN nu + SM mu)
+template <int SN, int SM, typename T, int NR>
+LT_D void acc_paths(M3<T>& a, T coef, const Gauge<T, NR>& A, const Gauge<T, NR>& B, const Geom& g, int par, int i,
+                    const int c[4], int mu)
+{
+    const int pn = par ^ (SN & 1), pm = SM & 1;
+    const int dmu = shift_offset(g, c, mu, SM);
+#pragma unroll 1
+    for (int n = 0; n < 3; ++n)
+    {
+        const int nu = n + (n >= mu ? 1 : 0);
+        const int inu = i + shift_offset(g, c, nu, SN), ind = i + shift_offset(g, c, nu, -SN);
+        M3<T> p = mul_nd(mul(A.ld(nu, par, i >> 1), B.ld(mu, pn, inu >> 1)), A.ld(nu, par ^ pm, (i + dmu) >> 1));
+        acc(p, mul(mul_dn(A.ld(nu, pn, ind >> 1), B.ld(mu, pn, ind >> 1)), A.ld(nu, pn ^ pm, (ind + dmu) >> 1)));
+#pragma unroll
+        for (int r = 0; r < 3; ++r)
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+            {
+                a.e[r][k].r += coef * p.e[r][k].r;
+                a.e[r][k].i += coef * p.e[r][k].i;
+            }
+    }
+}
+
+// The part along the link: E_mu(x) U_mu(x+mu)^dag + U_mu(x-mu)^dag E_mu(x-mu)
+template <typename T>
+LT_D void acc_rect_along(M3<T>& a, const Full<T>& E, int mu, int par, int s, int sdn, const M3<T>& u_up, const M3<T>& u_dn)
+{
+    acc(a, mul_nd(E.ld(mu, par, s), u_up));
+    acc(a, mul_dn(u_dn, E.ld(mu, par ^ 1, sdn)));
+}
+
+template <typename T, int NR>
+LT_D M3<T> staple_two_link(const Gauge<T, NR>& U, const RectFields<T, NR>& W, const Geom& g, int par, int i,
+                           const int c[4], int mu, T cp, T cr)
+{
+    M3<T> st = zero3<T>();
+    acc_paths<1, 1>(st, cp, U, U, g, par, i, c, mu);
+    acc_paths<2, 1>(st, cr, W.D, U, g, par, i, c, mu);
+    const int sup = (i + shift_offset(g, c, mu, 1)) >> 1, sdn = (i + shift_offset(g, c, mu, -1)) >> 1;
+    acc_rect_along(st, W.E, mu, par, i >> 1, sdn, U.ld(mu, par ^ 1, sup), U.ld(mu, par ^ 1, sdn));
+    return st;
+}
+
+// The same on two-row FP32 storage through the ring of staple_staged: six direction steps, the
+// plaquette paths (fields U, U) then the orthogonal rectangle paths (fields D, U, twice the
+// shift along nu), one path ahead; the three links of the part along the link follow the last
+// upper path into its slot.  u receives the link itself.
+template <int NT>
+LT_D M3<float> staple_two_link_staged(StapleRingT<NT>& r, const Gauge<float, 2>& U, const RectFields<float, 2>& W,
+                                      const Geom& g, int par, int i, int s, const int c[4], int mu, float cp, float cr,
+                                      M3<float>& u)
+{
+    const int op = par ^ 1;
+    const int dmu = step_up_rt(g, mu, c);
+    const int sup = (i + dmu) >> 1, sdn = (i + step_dn_rt(g, mu, c)) >> 1;
+    auto stage = [&](bool up, int n) {
+        const int sn = n < 3 ? 1 : 2, m = n < 3 ? n : n - 3, nu = m + (m >= mu ? 1 : 0);
+        const Gauge<float, 2>& A = n < 3 ? U : W.D;
+        const int pn = n < 3 ? op : par;
+        if (up)
+        {
+            const int inu = i + shift_offset(g, c, nu, sn);
+            stage_link(r, 0, 0, A.chunk(nu, par, 0) + s, U.vh);
+            stage_link(r, 0, 1, U.chunk(mu, pn, 0) + (inu >> 1), U.vh);
+            stage_link(r, 0, 2, A.chunk(nu, op, 0) + sup, U.vh);
+        }
+        else
+        {
+            const int ind = i + shift_offset(g, c, nu, -sn);
+            stage_link(r, 1, 0, A.chunk(nu, pn, 0) + (ind >> 1), U.vh);
+            stage_link(r, 1, 1, U.chunk(mu, pn, 0) + (ind >> 1), U.vh);
+            stage_link(r, 1, 2, A.chunk(nu, pn ^ 1, 0) + ((ind + dmu) >> 1), U.vh);
+        }
+    };
+    stage(true, 0);
+    cp_async_commit();
+    stage(false, 0);
+    cp_async_commit();
+    M3<float> st = zero3<float>();
+#pragma unroll 1
+    for (int n = 0; n < 6; ++n)
+    {
+        const float coef = n < 3 ? cp : cr;
+        cp_async_wait<1>();
+        acc_restored(st, coef,
+                     mul_nd_rows(mul_rows(staged_rows(r, 0, 0), staged_link(r, 0, 1)), staged_link(r, 0, 2)));
+        if (n < 5)
+            stage(true, n + 1);
+        else
+        {
+            stage_link(r, 0, 0, U.chunk(mu, par, 0) + s, U.vh);
+            stage_link(r, 0, 1, U.chunk(mu, op, 0) + sup, U.vh);
+            stage_link(r, 0, 2, U.chunk(mu, op, 0) + sdn, U.vh);
+        }
+        cp_async_commit();
+        cp_async_wait<1>();
+        acc_restored(st, coef,
+                     mul_rows(mul_dn_rows(staged_link(r, 1, 0), staged_link(r, 1, 1)), staged_link(r, 1, 2)));
+        if (n < 5) stage(false, n + 1);
+        cp_async_commit();
+    }
+    cp_async_wait<0>();
+    acc_rect_along(st, W.E, mu, par, s, sdn, staged_link(r, 0, 1), staged_link(r, 0, 2));
+    u = staged_link(r, 0, 0);
+    return st;
+}
+
+// D of every link
+template <typename T, int NR>
+__global__ void __launch_bounds__(kThreads) k_two_links(Gauge<T, NR> U, Gauge<T, NR> D, Geom g, int rev)
+{
+    pdl_release();
+    pdl_wait();
+    int mu, x;
+    if (!link_of_thread(g, mu, x, rev)) return;
+    const int par = x >= g.vh, s = x - par * g.vh;
+    int c[4];
+    const int i = site_coords(g, par, s, c);
+    const M3<T> b = U.ld(mu, par ^ 1, (i + step_up_rt(g, mu, c)) >> 1);
+    D.st(mu, par, s, NR == 2 ? mul_rows(U.ld_rows(mu, par, s), b) : mul(U.ld(mu, par, s), b));
+}
+
+// E of every link
+template <typename T, int NR>
+__global__ void __launch_bounds__(kThreads) k_rect_outer(Gauge<T, NR> U, RectFields<T, NR> W, Geom g, T cr, int rev)
+{
+    pdl_release();
+    pdl_wait();
+    int mu, x;
+    if (!link_of_thread(g, mu, x, rev)) return;
+    const int par = x >= g.vh, s = x - par * g.vh;
+    int c[4];
+    const int i = site_coords(g, par, s, c);
+    M3<T> e = zero3<T>();
+    acc_paths<1, 2>(e, cr, U, W.D, g, par, i, c, mu);
+    W.E.st(mu, par, s, e);
+}
+
+template <int Unused = 0>
+__global__ void __launch_bounds__(kStagedThreads, LT_MINB_STAGED)
+    k_rect_outer_staged(Gauge<float, 2> U, RectFields<float, 2> W, Geom g, float cr, int rev)
+{
+    __shared__ StapleRing ring;
+    pdl_release();
+    pdl_wait();
+    int mu, x;
+    if (!link_of_thread(g, mu, x, rev)) return;
+    const int par = x >= g.vh, s = x - par * g.vh, op = par ^ 1;
+    int c[4];
+    const int i = site_coords(g, par, s, c);
+    const int dmu2 = shift_offset(g, c, mu, 2);
+    auto stage = [&](bool up, int n) {
+        const int nu = n + (n >= mu ? 1 : 0);
+        if (up)
+        {
+            const int inu = i + step_up_rt(g, nu, c);
+            stage_link(ring, 0, 0, U.chunk(nu, par, 0) + s, U.vh);
+            stage_link(ring, 0, 1, W.D.chunk(mu, op, 0) + (inu >> 1), U.vh);
+            stage_link(ring, 0, 2, U.chunk(nu, par, 0) + ((i + dmu2) >> 1), U.vh);
+        }
+        else
+        {
+            const int ind = i + step_dn_rt(g, nu, c);
+            stage_link(ring, 1, 0, U.chunk(nu, op, 0) + (ind >> 1), U.vh);
+            stage_link(ring, 1, 1, W.D.chunk(mu, op, 0) + (ind >> 1), U.vh);
+            stage_link(ring, 1, 2, U.chunk(nu, op, 0) + ((ind + dmu2) >> 1), U.vh);
+        }
+    };
+    stage(true, 0);
+    cp_async_commit();
+    stage(false, 0);
+    cp_async_commit();
+    M3<float> e = zero3<float>();
+#pragma unroll 1
+    for (int n = 0; n < 3; ++n)
+    {
+        cp_async_wait<1>();
+        acc_restored(e, mul_nd_rows(mul_rows(staged_rows(ring, 0, 0), staged_link(ring, 0, 1)), staged_link(ring, 0, 2)));
+        if (n < 2) stage(true, n + 1);
+        cp_async_commit();
+        cp_async_wait<1>();
+        acc_restored(e, mul_rows(mul_dn_rows(staged_link(ring, 1, 0), staged_link(ring, 1, 1)), staged_link(ring, 1, 2)));
+        if (n < 2) stage(false, n + 1);
+        cp_async_commit();
+    }
+    W.E.st(mu, par, s, cr * e);
+}
+
 // The handle's gauge action on the device: Rectangular<1> (the plaquette staple alone, whatever
 // c_plaq) or Rectangular<2> (c_plaq StaplePlaq + c_rect StapleRect; rectangular_action.hpp:236-246)
 template <bool RECT, typename T, int NR>
@@ -776,6 +984,19 @@ LT_D M3<T> action_staple(const Gauge<T, NR>& U, const Geom& g, int par, int i, c
     }
     else
         return staple(U, g, par, i, c, mu);
+}
+
+// The action of a kernel over all links: Wilson, rectangles from the two-link fields W, or (where
+// there is no memory for those) rectangles path by path
+enum class Act { Wilson, TwoLink, Direct };
+template <Act ACT, typename T, int NR>
+LT_D M3<T> link_staple(const Gauge<T, NR>& U, const RectFields<T, NR>& W, const Geom& g, int par, int i, const int c[4],
+                       int mu, T cp, T cr)
+{
+    if constexpr (ACT == Act::TwoLink)
+        return staple_two_link(U, W, g, par, i, c, mu, cp, cr);
+    else
+        return action_staple<ACT == Act::Direct>(U, g, par, i, c, mu, cp, cr);
 }
 
 // Iterator::Checkerboard4 (iterators/iterators.hpp:141-166): for direction mu the links whose
@@ -1383,10 +1604,10 @@ template <int Unused = 0> __global__ void k_counter_add(uint64_t* c, uint64_t n)
 //   U'  <- exp(c_exp Z) U, Gram-Schmidt          (UpdateFields)
 // reading U from Uin and writing Uout (ping-pong), so all staples see the pre-stage field
 // exactly as the reference's separate Z and field sweeps do.
-template <typename T, int NR, bool RECT>
+template <typename T, int NR, Act ACT>
 __global__ void __launch_bounds__(kThreads, (LinkMinBlocks<T, NR>::value)) k_flow_stage(Gauge<T, NR> Uin, Gauge<T, NR> Uout, Alg<T> Z, Geom g,
-                                                         T c_old, T c_new, T c_exp, int read_z, int write_z, T cp, T cr,
-                                                         int rev)
+                                                         T c_old, T c_new, T c_exp, int read_z, int write_z,
+                                                         RectFields<T, NR> W, T cp, T cr, int rev)
 {
     pdl_release();
     pdl_wait();
@@ -1396,7 +1617,7 @@ __global__ void __launch_bounds__(kThreads, (LinkMinBlocks<T, NR>::value)) k_flo
     int c[4];
     int i = site_coords(g, par, s, c);
     M3<T> u = Uin.ld(mu, par, s);
-    M3<T> st = action_staple<RECT>(Uin, g, par, i, c, mu, cp, cr);
+    M3<T> st = link_staple<ACT>(Uin, W, g, par, i, c, mu, cp, cr);
     A8<T> a = algebra8(mul_nd(st, u));
     A8<T> z;
     if (read_z)
@@ -1414,15 +1635,15 @@ __global__ void __launch_bounds__(kThreads, (LinkMinBlocks<T, NR>::value)) k_flo
     Uout.st(mu, par, s, exp_update<T, NR>(unpack_ah(z), c_exp, u));
 }
 
-// k_flow_stage (Wilson action) on two-row FP32 storage with the staged staple; Z of the link
+// k_flow_stage on two-row FP32 storage with the staged staple (ACT: Wilson or TwoLink); Z of the link
 // is read before the staple so that its loads are in flight meanwhile
 #ifndef LT_MINB_FLOW_STAGED
 #define LT_MINB_FLOW_STAGED 5
 #endif
-template <int Unused = 0>
+template <Act ACT>
 __global__ void __launch_bounds__(4 * kSitesPerBlock, LT_MINB_FLOW_STAGED)
     k_flow_stage_staged(Gauge<float, 2> Uin, Gauge<float, 2> Uout, Alg<float> Z, Geom g, float c_old, float c_new,
-                        float c_exp, int read_z, int write_z, int rev)
+                        float c_exp, int read_z, int write_z, RectFields<float, 2> W, float cp, float cr, int rev)
 {
     static_assert(4 * kSitesPerBlock == kStagedThreads, "one ring slot per thread");
     __shared__ StapleRing ring;
@@ -1437,7 +1658,8 @@ __global__ void __launch_bounds__(4 * kSitesPerBlock, LT_MINB_FLOW_STAGED)
     if (read_z)
         z = Z.ld(mu, par, s);
     M3<float> u;
-    const M3<float> st = staple_staged<true>(ring, Uin, g, par, i, s, c, mu, u);
+    const M3<float> st = ACT == Act::TwoLink ? staple_two_link_staged(ring, Uin, W, g, par, i, s, c, mu, cp, cr, u)
+                                             : staple_staged<true>(ring, Uin, g, par, i, s, c, mu, u);
     const A8<float> a = algebra8(mul_nd(st, u));
 #pragma unroll
     for (int k = 0; k < 8; ++k) z.a[k] = read_z ? c_old * z.a[k] + c_new * a.a[k] : c_new * a.a[k];
@@ -1462,12 +1684,12 @@ __global__ void __launch_bounds__(4 * kSitesPerBlock, LT_MINB_FLOW_STAGED)
 #ifndef LT_MINB_FLOW_FORCE_RECT_F32C
 #define LT_MINB_FLOW_FORCE_RECT_F32C 6
 #endif
-template <typename T, int NR, bool RECT> struct FlowForceMinBlocks
+template <typename T, int NR, Act ACT> struct FlowForceMinBlocks
 {
-    static constexpr int value = (sizeof(T) == 4 && NR == 2 && RECT) ? LT_MINB_FLOW_FORCE_RECT_F32C : 1;
+    static constexpr int value = (sizeof(T) == 4 && NR == 2 && ACT == Act::Direct) ? LT_MINB_FLOW_FORCE_RECT_F32C : 1;
 };
-template <typename T, int NR, bool RECT>
-__global__ void __launch_bounds__(kThreads, (FlowForceMinBlocks<T, NR, RECT>::value)) k_flow_force(Gauge<T, NR> U, Alg<T> X, Geom g, T cp, T cr, int rev)
+template <typename T, int NR, Act ACT>
+__global__ void __launch_bounds__(kThreads, (FlowForceMinBlocks<T, NR, ACT>::value)) k_flow_force(Gauge<T, NR> U, Alg<T> X, Geom g, RectFields<T, NR> W, T cp, T cr, int rev)
 {
     pdl_release();
     pdl_wait();
@@ -1477,7 +1699,25 @@ __global__ void __launch_bounds__(kThreads, (FlowForceMinBlocks<T, NR, RECT>::va
     int c[4];
     const int i = site_coords(g, par, s, c);
     const M3<T> u = U.ld(mu, par, s);
-    X.st(mu, par, s, algebra8(mul_nd(action_staple<RECT>(U, g, par, i, c, mu, cp, cr), u)));
+    X.st(mu, par, s, algebra8(mul_nd(link_staple<ACT>(U, W, g, par, i, c, mu, cp, cr), u)));
+}
+
+// k_flow_force with the two-link rectangles on two-row FP32 storage
+template <int Unused = 0>
+__global__ void __launch_bounds__(4 * kSitesPerBlock, LT_MINB_STAGED)
+    k_flow_force_staged(Gauge<float, 2> U, Alg<float> X, Geom g, RectFields<float, 2> W, float cp, float cr, int rev)
+{
+    __shared__ StapleRing ring;
+    pdl_release();
+    pdl_wait();
+    int mu, x;
+    if (!link_of_thread(g, mu, x, rev)) return;
+    const int par = x >= g.vh, s = x - par * g.vh;
+    int c[4];
+    const int i = site_coords(g, par, s, c);
+    M3<float> u;
+    const M3<float> st = staple_two_link_staged(ring, U, W, g, par, i, s, c, mu, cp, cr, u);
+    X.st(mu, par, s, algebra8(mul_nd(st, u)));
 }
 
 // The second half of a split flow stage: Z <- c_old Z + c_new X, U' = exp(c_exp Z) U, with
@@ -1998,15 +2238,15 @@ __global__ void __launch_bounds__(kRedThreads) k_polyakov(Gauge<T, NR> Ust, Geom
 // ---------------------------------------------------------------- HMC
 // HMC momentum kick P += eps * (beta/6 Algebra(st U^dag) + F)  (updates/hmc_gauge.hpp:450-464,
 // updates/hmc_metadynamics.hpp:441-459).  With P = null the force itself is written to F_out.
-template <typename T, int NR, bool RECT>
-__global__ void __launch_bounds__(kThreads, (LinkMinBlocks<T, NR>::value)) k_momenta(Gauge<T, NR> U, Alg<T> P, Alg<T> F, Geom g, T coef, T eps, int use_f, T cp, T cr)
+template <typename T, int NR, Act ACT>
+__global__ void __launch_bounds__(kThreads, (LinkMinBlocks<T, NR>::value)) k_momenta(Gauge<T, NR> U, Alg<T> P, Alg<T> F, Geom g, T coef, T eps, int use_f, RectFields<T, NR> W, T cp, T cr)
 {
     int mu, x;
     if (!link_of_thread(g, mu, x)) return;
     int par = x >= g.vh, s = x - par * g.vh;
     int c[4];
     int i = site_coords(g, par, s, c);
-    M3<T> st = action_staple<RECT>(U, g, par, i, c, mu, cp, cr);
+    M3<T> st = link_staple<ACT>(U, W, g, par, i, c, mu, cp, cr);
     A8<T> a = algebra8(mul_nd(st, U.ld(mu, par, s)));
     A8<T> p = P.ld(mu, par, s);
     if (use_f)
@@ -2023,11 +2263,12 @@ __global__ void __launch_bounds__(kThreads, (LinkMinBlocks<T, NR>::value)) k_mom
     P.st(mu, par, s, p);
 }
 
-// k_momenta (Wilson action) on two-row FP32 storage with the staged staple; P (and F) of the
-// link are read before the staple so that their loads are in flight meanwhile
-template <int Unused = 0>
+// k_momenta on two-row FP32 storage with the staged staple (ACT: Wilson or TwoLink); P (and F) of
+// the link are read before the staple so that their loads are in flight meanwhile
+template <Act ACT>
 __global__ void __launch_bounds__(4 * kSitesPerBlock, LT_MINB_FLOW_STAGED)
-    k_momenta_staged(Gauge<float, 2> U, Alg<float> P, Alg<float> F, Geom g, float coef, float eps, int use_f)
+    k_momenta_staged(Gauge<float, 2> U, Alg<float> P, Alg<float> F, Geom g, float coef, float eps, int use_f,
+                     RectFields<float, 2> W, float cp, float cr)
 {
     __shared__ StapleRing ring;
     int mu, x;
@@ -2039,7 +2280,8 @@ __global__ void __launch_bounds__(4 * kSitesPerBlock, LT_MINB_FLOW_STAGED)
     if (use_f)
         f = F.ld(mu, par, s);
     M3<float> u;
-    const M3<float> st = staple_staged<true>(ring, U, g, par, i, s, c, mu, u);
+    const M3<float> st = ACT == Act::TwoLink ? staple_two_link_staged(ring, U, W, g, par, i, s, c, mu, cp, cr, u)
+                                             : staple_staged<true>(ring, U, g, par, i, s, c, mu, u);
     const A8<float> a = algebra8(mul_nd(st, u));
 #pragma unroll
     for (int k = 0; k < 8; ++k) p.a[k] += use_f ? eps * (coef * a.a[k] + f.a[k]) : eps * coef * a.a[k];

@@ -341,6 +341,27 @@ template <typename T> LT_HD void acc_restored(M3<T>& a, const M3<T>& p)
     a.e[2][2] = acc_conj_cross(a.e[2][2], p.e[0][0], p.e[1][1], p.e[0][1], p.e[1][0]);
 }
 
+// a += s p for such a p
+template <typename T> LT_HD void acc_restored(M3<T>& a, T s, const M3<T>& p)
+{
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+        {
+            a.e[i][j].r += s * p.e[i][j].r;
+            a.e[i][j].i += s * p.e[i][j].i;
+        }
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+    {
+        const int k = (j + 1) % 3, l = (j + 2) % 3;
+        const cx<T> c = conj_cross(p.e[0][k], p.e[1][l], p.e[0][l], p.e[1][k]);
+        a.e[2][j].r += s * c.r;
+        a.e[2][j].i += s * c.i;
+    }
+}
+
 template <typename T> LT_HD void restore_last_row(M3<T>& a)
 {
     a.e[2][0] = conj_cross(a.e[0][1], a.e[1][2], a.e[0][2], a.e[1][1]);
