@@ -356,14 +356,19 @@ public:
     void sweep4(const Ctx& c, void* U, int op, int mu, int sub, double prefactor, uint64_t counter, uint64_t seed,
                 int max_iter) const override
     {
+        if (c.rect)
+        {
+            launch_chained(op == 0 ? k_sweep4_rect<T, NR, 0> : k_sweep4_rect<T, NR, 1>, nblocks(c.g.V / 4, 32),
+                           32 * kRectWarps, c.stream, gauge(U, c.g), c.g, mu, sub, (T)prefactor, counter, (uint32_t)seed,
+                           (uint32_t)(seed >> 32), max_iter, c.status, (T)c.cp, (T)c.cr, next_order(c));
+            return;
+        }
         const int nb = nblocks(c.g.V / 4, kThreads);
         if (op == 0)
-            launch_chained(c.rect ? k_heatbath4<T, NR, true> : k_heatbath4<T, NR, false>, nb, kThreads, c.stream,
-                           gauge(U, c.g), c.g, mu, sub, (T)prefactor, counter, (uint32_t)seed, (uint32_t)(seed >> 32),
-                           max_iter, c.status, (T)c.cp, (T)c.cr, next_order(c));
+            launch_chained(k_heatbath4<T, NR>, nb, kThreads, c.stream, gauge(U, c.g), c.g, mu, sub, (T)prefactor, counter,
+                           (uint32_t)seed, (uint32_t)(seed >> 32), max_iter, c.status, next_order(c));
         else
-            launch_chained(c.rect ? k_overrelax4<T, NR, true> : k_overrelax4<T, NR, false>, nb, kThreads, c.stream,
-                           gauge(U, c.g), c.g, mu, sub, (T)c.cp, (T)c.cr, next_order(c));
+            launch_chained(k_overrelax4<T, NR>, nb, kThreads, c.stream, gauge(U, c.g), c.g, mu, sub, next_order(c));
     }
     void alg_axpby(const Ctx& c, void* P, const void* F, double a, double b) const override
     {

@@ -51,16 +51,6 @@ template <typename T, int NR> struct Cb4MinBlocks
 {
     static constexpr int value = (sizeof(T) == 4 && NR == 2) ? 5 : MinBlocks<T>::sweep;
 };
-// Checkerboard4 sub-sweeps with rectangles: 4 blocks of 128 per SM on two-row FP32 storage
-// (128 registers, 28 bytes spilled; 7 % faster than 3 blocks at 157 registers), no cap for
-// the others (FP64 spills above 1 KB per thread at 4 blocks)
-#ifndef LT_MINB_RECT_F32C
-#define LT_MINB_RECT_F32C 4
-#endif
-template <typename T, int NR> struct RectMinBlocks
-{
-    static constexpr int value = (sizeof(T) == 4 && NR == 2) ? LT_MINB_RECT_F32C : 1;
-};
 // link-parallel kernels: two-row FP32 storage has its own setting
 template <typename T, int NR> struct LinkMinBlocks
 {
@@ -1116,9 +1106,9 @@ __global__ void __launch_bounds__(kStagedThreads, LT_MINB_STAGED) k_overrelax_st
     U.st(mu, par, s, u);
 }
 
-// One (mu, sublattice) sub-sweep of Iterator::Checkerboard4 with the handle's action
-template <typename T, int NR, bool RECT>
-__global__ void __launch_bounds__(kThreads, (RECT ? RectMinBlocks<T, NR>::value : Cb4MinBlocks<T, NR>::value)) k_overrelax4(Gauge<T, NR> U, Geom g, int mu, int sub, T cp, T cr, int rev)
+// One (mu, sublattice) sub-sweep of Iterator::Checkerboard4 with the Wilson action
+template <typename T, int NR>
+__global__ void __launch_bounds__(kThreads, (Cb4MinBlocks<T, NR>::value)) k_overrelax4(Gauge<T, NR> U, Geom g, int mu, int sub, int rev)
 {
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     pdl_release();
@@ -1128,7 +1118,7 @@ __global__ void __launch_bounds__(kThreads, (RECT ? RectMinBlocks<T, NR>::value 
     int c[4];
     const int i = cb4_site(g, mu, sub, k, c);
     const int par = (c[0] + c[1] + c[2] + c[3]) & 1, s = i >> 1;
-    const M3<T> st = action_staple<RECT>(U, g, par, i, c, mu, cp, cr);
+    const M3<T> st = staple(U, g, par, i, c, mu);
     M3<T> u = U.ld(mu, par, s);
     or_apply<T, NR>(u, st);
     U.st(mu, par, s, u);
@@ -1325,11 +1315,11 @@ __global__ void __launch_bounds__(kStagedThreads, LT_MINB_STAGED) k_heatbath_sta
     hb_core_u(U, mu, par, s, i, u, st, prefactor, counter, k0, k1, max_iter, status);
 }
 
-// One (mu, sublattice) sub-sweep of Iterator::Checkerboard4 with the handle's action
-template <typename T, int NR, bool RECT>
-__global__ void __launch_bounds__(kThreads, (RECT ? RectMinBlocks<T, NR>::value : Cb4MinBlocks<T, NR>::value)) k_heatbath4(Gauge<T, NR> U, Geom g, int mu, int sub, T prefactor,
+// One (mu, sublattice) sub-sweep of Iterator::Checkerboard4 with the Wilson action
+template <typename T, int NR>
+__global__ void __launch_bounds__(kThreads, (Cb4MinBlocks<T, NR>::value)) k_heatbath4(Gauge<T, NR> U, Geom g, int mu, int sub, T prefactor,
                                                         uint64_t counter, uint32_t k0, uint32_t k1, int max_iter,
-                                                        unsigned* status, T cp, T cr, int rev)
+                                                        unsigned* status, int rev)
 {
     int k = blockIdx.x * blockDim.x + threadIdx.x;
     pdl_release();
@@ -1339,8 +1329,7 @@ __global__ void __launch_bounds__(kThreads, (RECT ? RectMinBlocks<T, NR>::value 
     int c[4];
     const int i = cb4_site(g, mu, sub, k, c);
     const int par = (c[0] + c[1] + c[2] + c[3]) & 1;
-    hb_core(U, mu, par, i >> 1, i, action_staple<RECT>(U, g, par, i, c, mu, cp, cr), prefactor, counter, k0, k1,
-            max_iter, status);
+    hb_core(U, mu, par, i >> 1, i, staple(U, g, par, i, c, mu), prefactor, counter, k0, k1, max_iter, status);
 }
 
 // Cabibbo-Marinari update of U_mu at site i (checkerboard index s) against the staple st
@@ -1371,6 +1360,128 @@ LT_D void hb_core_u(const Gauge<T, NR>& U, int mu, int par, int s, int i, M3<T> 
     gram_schmidt<T, NR == 3>(u);
     U.st(mu, par, s, u);
     if (capped && status) atomicOr(status, kStatusHbCap);
+}
+
+// ---------------------------------------------------------------- rectangle sweeps
+// One (mu, sublattice) sub-sweep of Iterator::Checkerboard4 with a Rectangular<2> action: nine
+// warps share 32 links.  For each direction nu one warp takes the paths orthogonal to the link
+// (plaquettes and 1x2 loops, which share their outer links), one the 2x1 loops that leave x along
+// mu and one those that arrive along mu; the nine partial staples meet in shared memory, each
+// warp sums one matrix element, and the first warp updates the 32 links.
+// A sub-sweep has only V/4 links: one thread a link left a 16^4 lattice with a single block of four
+// warps per SM, each waiting for its own chain of 78 products and 102 link loads.  Shared, a
+// warp's chain is 7 or 8 products (66 a link), the loads of nine warps are in flight together, and
+// the partial staples need far fewer registers than the whole one.  Per launch, one thread a link
+// and shared: FP64 16^4 44.2 and 30.0 us (overrelaxation), 53.0 and 42.7 (heatbath), 24^4 161 and 148;
+// two-row FP32 8^4 25.1 and 6.3, 16^4 48.1 and 15.0, 32^4 207 and 198.  In FP64 the launch is bound by the
+// links that come from L2 (90 a link, 144 bytes each, half of every 32-byte sector for the stride-2 sites).
+constexpr int kRectWarps = 9;
+
+// The three-link path a b c of SU(3) links; two-row storage multiplies two rows and rebuilds the third
+template <int NR, bool DC, typename T> LT_D M3<T> path3(const M3<T>& a, const M3<T>& b, const M3<T>& c)
+{
+    if (NR == 2)
+    {
+        M3<T> p = mul_rows(a, b);
+        p = DC ? mul_nd_rows(p, c) : mul_rows(p, c);
+        restore_last_row(p);
+        return p;
+    }
+    const M3<T> p = mul(a, b);
+    return DC ? mul_nd(p, c) : mul(p, c);
+}
+
+template <typename T, int NR>
+LT_D M3<T> rect_partial(const Gauge<T, NR>& U, const Geom& g, int par, int i, const int c[4], int mu, int nu, int kind,
+                        T cp, T cr)
+{
+    auto at = [&](int dm, int dn) { return site_at(g, i, c, mu, dm, nu, dn) >> 1; };
+    auto L = [&](int d, int dm, int dn) { return U.ld(d, par ^ ((dm + dn) & 1), at(dm, dn)); };
+    M3<T> r;
+    if (kind == 0)
+    {
+        // U_nu(x) [cp U_mu(x+nu) + cr U_nu(x+nu) U_mu(x+2nu) U_nu(x+mu+nu)^dag] U_nu(x+mu)^dag
+        M3<T> t = cr * path3<NR, true>(L(nu, 0, 1), L(mu, 0, 2), L(nu, 1, 1));
+        acc(t, cp * L(mu, 0, 1));
+        r = mul_nd(mul(L(nu, 0, 0), t), L(nu, 1, 0));
+        // U_nu(x-nu)^dag [cp U_mu(x-nu) + cr U_nu(x-2nu)^dag U_mu(x-2nu) U_nu(x+mu-2nu)] U_nu(x+mu-nu)
+        t = cr * path3<NR, false>(adj(L(nu, 0, -2)), L(mu, 0, -2), L(nu, 1, -2));
+        acc(t, cp * L(mu, 0, -1));
+        acc(r, mul(mul_dn(L(nu, 0, -1), t), L(nu, 1, -1)));
+        return r;
+    }
+    // the four-link paths over and under the link, from x (kind 1) or from x - mu (kind 2), closed
+    // with the link along mu that they share
+    const int m0 = kind == 1 ? 0 : -1;
+    if (NR == 2)
+    {
+        M3<T> p = mul_nd_rows(mul_rows(mul_rows(L(nu, m0, 0), L(mu, m0, 1)), L(mu, m0 + 1, 1)), L(nu, m0 + 2, 0));
+        r = zero3<T>();
+        acc_restored(r, p);
+        p = mul_rows(mul_rows(mul_dn_rows(L(nu, m0, -1), L(mu, m0, -1)), L(mu, m0 + 1, -1)), L(nu, m0 + 2, -1));
+        acc_restored(r, p);
+    }
+    else
+    {
+        r = mul_nd(mul(mul(L(nu, m0, 0), L(mu, m0, 1)), L(mu, m0 + 1, 1)), L(nu, m0 + 2, 0));
+        acc(r, mul(mul(mul_dn(L(nu, m0, -1), L(mu, m0, -1)), L(mu, m0 + 1, -1)), L(nu, m0 + 2, -1)));
+    }
+    return cr * (kind == 1 ? mul_nd(r, L(mu, 1, 0)) : mul_dn(L(mu, -1, 0), r));
+}
+
+// Blocks per SM asked for, measured at 8^4, 16^4, 24^4 and 32^4: FP64 overrelaxation one (168 registers; two
+// spill 640 bytes: 8.5 against 13.5 us at 8^4, 148 against 173 at 24^4), FP64 heatbath two (its first warp's
+// update overlaps the other block's paths: 198 against 220 us at 24^4); FP32 two and three (two-row links at
+// 32^4: heatbath 195 us with three, 217 with two; overrelaxation at 16^4 15.0 with two, 17.6 with three)
+template <typename T, int OP> struct RectMinBlocks
+{
+    static constexpr int value = (sizeof(T) == 4 ? 2 : 1) + (OP == 0 ? 1 : 0);
+};
+
+// OP: 0 heatbath, 1 overrelaxation
+template <typename T, int NR, int OP>
+__global__ void __launch_bounds__(32 * kRectWarps, (RectMinBlocks<T, OP>::value))
+    k_sweep4_rect(Gauge<T, NR> U, Geom g, int mu, int sub, T prefactor, uint64_t counter, uint32_t k0, uint32_t k1,
+                  int max_iter, unsigned* status, T cp, T cr, int rev)
+{
+    __shared__ cx<T> part[kRectWarps][9][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, n = g.V >> 2;
+    pdl_release();
+    pdl_wait();
+    int k = blockIdx.x * 32 + lane;
+    const bool ok = k < n;
+    if (!ok) k = n - 1;   // the last block's spare lanes follow the last link and store nothing
+    if (rev) k = n - 1 - k;
+    int c[4];
+    const int i = cb4_site(g, mu, sub, k, c);
+    const int par = (c[0] + c[1] + c[2] + c[3]) & 1, s = i >> 1;
+    const int dir = w / 3;
+    {
+        const M3<T> p = rect_partial(U, g, par, i, c, mu, dir + (dir >= mu ? 1 : 0), w - 3 * dir, cp, cr);
+#pragma unroll
+        for (int e = 0; e < 9; ++e) part[w][e][lane] = p.e[e / 3][e % 3];
+    }
+    __syncthreads();
+    {
+        // element w of the sum; only this warp reads and writes it
+        cx<T> sum = part[0][w][lane];
+#pragma unroll
+        for (int q = 1; q < kRectWarps; ++q) sum = sum + part[q][w][lane];
+        part[0][w][lane] = sum;
+    }
+    __syncthreads();
+    if (w != 0 || !ok) return;
+    M3<T> st;
+#pragma unroll
+    for (int e = 0; e < 9; ++e) st.e[e / 3][e % 3] = part[0][e][lane];
+    if (OP == 0)
+        hb_core(U, mu, par, s, i, st, prefactor, counter, k0, k1, max_iter, status);
+    else
+    {
+        M3<T> u = U.ld(mu, par, s);
+        or_apply<T, NR>(u, st);
+        U.st(mu, par, s, u);
+    }
 }
 
 // ---------------------------------------------------------------- batched sweeps
