@@ -1362,6 +1362,70 @@ LT_D void hb_core_u(const Gauge<T, NR>& U, int mu, int par, int s, int i, M3<T> 
     if (capped && status) atomicOr(status, kStatusHbCap);
 }
 
+// ---------------------------------------------------------------- split sweeps
+// One (mu, parity) sub-sweep with six warps sharing 32 links: each warp multiplies out one of the
+// six staple paths, the paths meet in shared memory and are summed in the order of staple(), and the
+// first warp updates the links.  Same products and sums as k_overrelax and k_heatbath, bit for bit.
+// One thread a link, an 8^4 lattice has 16 blocks and every thread waits for its whole chain; shared, a
+// launch takes (one thread a link, shared) FP64 8^4 6.7 and 4.0 us overrelaxation, 11.0 and 8.5 heatbath;
+// 12^4 11.3 and 6.0, 16.8 and 12.2; FP32 8^4 6.4 and 3.1, 7.4 and 4.0; 16^4 11.5 and 7.3, 13.4 and 9.5.  Once
+// every SM has several blocks the idle warps of the update cost more than the shorter chain gives
+// (FP64 16^4 12.4 and 13.5, 17.9 and 25.5; FP32 32^4 75 and 93), which sets the rule of split_sweep.
+template <typename T, int NR, int OP, int MINB>   // OP: 0 heatbath, 1 overrelaxation
+__global__ void __launch_bounds__(192, MINB)
+    k_sweep_split(Gauge<T, NR> U, Geom g, int mu, int par, T prefactor, uint64_t counter, uint32_t k0, uint32_t k1,
+                  int max_iter, unsigned* status, int rev)
+{
+    static_assert(NR == 3, "paths summed as full matrices");
+    __shared__ cx<T> part[6][9][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    int s = blockIdx.x * 32 + lane;
+    const bool ok = s < g.vh;
+    if (!ok) s = g.vh - 1;   // spare lanes of the last block follow the last link and store nothing
+    if (rev) s = g.vh - 1 - s;
+    int c[4];
+    const int i = site_coords(g, par, s, c), op = par ^ 1;
+    pdl_release();
+    pdl_wait();
+    {
+        const int n = w >> 1, nu = n + (n >= mu ? 1 : 0), dmu = step_up_rt(g, mu, c);
+        M3<T> p;
+        if (w & 1)
+        {
+            const int ind = i + step_dn_rt(g, nu, c);
+            p = mul(mul_dn(U.ld(nu, op, ind >> 1), U.ld(mu, op, ind >> 1)), U.ld(nu, par, (ind + dmu) >> 1));
+        }
+        else
+        {
+            const int inu = i + step_up_rt(g, nu, c);
+            p = mul_nd(mul(U.ld(nu, par, s), U.ld(mu, op, inu >> 1)), U.ld(nu, op, (i + dmu) >> 1));
+        }
+#pragma unroll
+        for (int e = 0; e < 9; ++e) part[w][e][lane] = p.e[e / 3][e % 3];
+    }
+    __syncthreads();
+    for (int e = w; e < 9; e += 6)   // only this warp reads and writes the element
+    {
+        cx<T> sum = mkc<T>(0, 0);
+#pragma unroll
+        for (int n = 0; n < 3; ++n) sum = sum + (part[2 * n][e][lane] + part[2 * n + 1][e][lane]);
+        part[0][e][lane] = sum;
+    }
+    __syncthreads();
+    if (w != 0 || !ok) return;
+    M3<T> st;
+#pragma unroll
+    for (int e = 0; e < 9; ++e) st.e[e / 3][e % 3] = part[0][e][lane];
+    if (OP == 0)
+        hb_core(U, mu, par, s, i, st, prefactor, counter, k0, k1, max_iter, status);
+    else
+    {
+        M3<T> u = U.ld(mu, par, s);
+        or_apply<T, NR>(u, st);
+        U.st(mu, par, s, u);
+    }
+}
+
 // ---------------------------------------------------------------- rectangle sweeps
 // One (mu, sublattice) sub-sweep of Iterator::Checkerboard4 with a Rectangular<2> action: nine
 // warps share 32 links.  For each direction nu one warp takes the paths orthogonal to the link
