@@ -115,7 +115,7 @@ public:
     }
     void to_aos(const Ctx& c, const void* U, double* aos) const override
     {
-        k_to_aos<T, NR><<<nblocks(4LL * c.g.V, 256), 256, 0, c.stream>>>(gauge(U, c.g), c.g, aos);
+        k_to_aos<T, NR><<<nblocks(c.g.V, kAosSites), 256, 0, c.stream>>>(gauge(U, c.g), c.g, aos);
     }
     void alg_from_aos(const Ctx& c, void* P, const double* aos) const override
     {
@@ -123,7 +123,7 @@ public:
     }
     void alg_to_aos(const Ctx& c, const void* P, double* aos) const override
     {
-        k_alg_to_aos<T><<<nblocks(4LL * c.g.V, 256), 256, 0, c.stream>>>(alg(P, c.g), c.g, aos);
+        k_alg_to_aos<T><<<nblocks(c.g.V, kAosSites), 256, 0, c.stream>>>(alg(P, c.g), c.g, aos);
     }
     void set_unit(const Ctx& c, void* U) const override
     {
