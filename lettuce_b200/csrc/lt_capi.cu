@@ -11,6 +11,7 @@
 #include <new>
 #include <string>
 #include <thread>
+#include <unordered_map>
 #include <vector>
 #if defined(__SSE2__)
 #include <emmintrin.h>
@@ -35,6 +36,94 @@ int cuda_error(cudaError_t e, const char* what)
     return e == cudaErrorMemoryAllocation ? LT_ERR_NOMEM : LT_ERR_CUDA;
 }
 
+namespace {
+struct DevStore
+{
+    std::unordered_map<void*, size_t> size;             // every buffer handed out or kept
+    std::unordered_multimap<size_t, void*> kept;        // buffers of no handle, by size
+    size_t kept_bytes = 0, most = 0;
+    int handles = 0;
+
+    void give_back()
+    {
+        for (auto& k : kept)
+        {
+            size.erase(k.second);
+            cudaFree(k.second);
+        }
+        kept.clear();
+        kept_bytes = 0;
+    }
+};
+std::mutex g_store_mutex;
+// by device; never destroyed, so that handles freed at process exit still find it
+std::unordered_map<int, DevStore>& stores()
+{
+    static auto* s = new std::unordered_map<int, DevStore>();
+    return *s;
+}
+} // namespace
+
+cudaError_t dev_alloc(int device, void** p, size_t bytes)
+{
+    std::lock_guard<std::mutex> lk(g_store_mutex);
+    DevStore& st = stores()[device];
+    const auto k = st.kept.find(bytes);
+    if (k != st.kept.end())
+    {
+        *p = k->second;
+        st.kept.erase(k);
+        st.kept_bytes -= bytes;
+        return cudaSuccess;
+    }
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaSuccess && st.kept_bytes)
+    {
+        (void)cudaGetLastError();
+        st.give_back();
+        e = cudaMalloc(p, bytes);
+    }
+    if (e == cudaSuccess) st.size[*p] = bytes;
+    else *p = nullptr;
+    return e;
+}
+
+void dev_free(int device, void* p)
+{
+    std::lock_guard<std::mutex> lk(g_store_mutex);
+    DevStore& st = stores()[device];
+    const auto k = st.size.find(p);
+    if (k == st.size.end()) return;
+    if (!st.most)
+    {
+        size_t avail = 0, total = 0;
+        if (cudaMemGetInfo(&avail, &total) == cudaSuccess) st.most = total / 8;
+        else (void)cudaGetLastError();
+    }
+    const size_t bytes = k->second;
+    if (st.kept_bytes + bytes > st.most)
+    {
+        st.size.erase(k);
+        cudaFree(p);
+        return;
+    }
+    st.kept.emplace(bytes, p);
+    st.kept_bytes += bytes;
+}
+
+void dev_handle_created(int device)
+{
+    std::lock_guard<std::mutex> lk(g_store_mutex);
+    ++stores()[device].handles;
+}
+
+void dev_handle_gone(int device)
+{
+    std::lock_guard<std::mutex> lk(g_store_mutex);
+    DevStore& st = stores()[device];
+    if (--st.handles == 0) st.give_back();
+}
+
 } // namespace lt
 
 namespace {
@@ -48,8 +137,16 @@ int check_h(const lt_lattice* h, const char* fn)
 int ensure(lt_lattice* h, void** p, size_t bytes)
 {
     if (*p) return LT_OK;
-    LT_CK(cudaMalloc(p, bytes));
+    LT_CK(lt::dev_alloc(h->device, p, bytes));
     return LT_OK;
+}
+
+// Scratch that a call can do without: false, with no error left behind, if there is no memory
+bool try_ensure(lt_lattice* h, void** p, size_t bytes)
+{
+    if (*p || lt::dev_alloc(h->device, p, bytes) == cudaSuccess) return true;
+    (void)cudaGetLastError();
+    return false;
 }
 
 // The scratch fields of a rectangle force over all links.  On the largest lattices there may be no
@@ -57,12 +154,9 @@ int ensure(lt_lattice* h, void** p, size_t bytes)
 void ensure_rect(lt_lattice* h)
 {
     if (h->rectE) return;
-    if (cudaMalloc(&h->rectD, h->be->gauge_bytes(h->g)) == cudaSuccess &&
-        cudaMalloc(&h->rectE, h->be->full_bytes(h->g)) == cudaSuccess)
-        return;
-    (void)cudaGetLastError();
-    if (h->rectD) cudaFree(h->rectD);
-    h->rectD = h->rectE = nullptr;
+    if (try_ensure(h, &h->rectD, h->be->gauge_bytes(h->g)) && try_ensure(h, &h->rectE, h->be->full_bytes(h->g))) return;
+    if (h->rectD) lt::dev_free(h->device, h->rectD);
+    h->rectD = nullptr;
 }
 
 int ensure_aos(lt_lattice* h) { return ensure(h, (void**)&h->d_aos, (size_t)4 * h->g.V * 18 * sizeof(double)); }
@@ -179,13 +273,13 @@ int metad_forward(lt_lattice* h, double rho, int n_stout)
     while ((int)h->levels.size() < n_stout)
     {
         void* p = nullptr;
-        LT_CK(cudaMalloc(&p, h->be->gauge_bytes(h->g)));
+        LT_CK(lt::dev_alloc(h->device, &p, h->be->gauge_bytes(h->g)));
         h->levels.push_back(p);
     }
     while ((int)h->staples.size() < n_stout)
     {
         void* p = nullptr;
-        LT_CK(cudaMalloc(&p, h->be->full_bytes(h->g)));
+        LT_CK(lt::dev_alloc(h->device, &p, h->be->full_bytes(h->g)));
         h->staples.push_back(p);
     }
     const lt::Ctx c = h->ctx();
@@ -823,12 +917,14 @@ int lt_create(const int ext[4], int prec, lt_lattice** out)
     h->be = be;
     cudaError_t e = cudaGetDevice(&h->device);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaMalloc(&h->U, be->gauge_bytes(h->g));
-    if (e == cudaSuccess) e = cudaMalloc((void**)&h->partials, sizeof(double) * lt::kNumSlots * lt::kRedBlocks);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&h->results, sizeof(double) * lt::kNumSlots);
+    lt::dev_handle_created(h->device);
+    if (e == cudaSuccess) e = lt::dev_alloc(h->device, &h->U, be->gauge_bytes(h->g));
+    if (e == cudaSuccess)
+        e = lt::dev_alloc(h->device, (void**)&h->partials, sizeof(double) * lt::kNumSlots * lt::kRedBlocks);
+    if (e == cudaSuccess) e = lt::dev_alloc(h->device, (void**)&h->results, sizeof(double) * lt::kNumSlots);
     if (e == cudaSuccess) e = cudaMallocHost((void**)&h->h_results, sizeof(double) * lt::kNumSlots);
     // status[0]: the status word; status[1]: scratch of lt_check_links; status[2]: of lt_load_bmw
-    if (e == cudaSuccess) e = cudaMalloc((void**)&h->status, 4 * sizeof(unsigned));
+    if (e == cudaSuccess) e = lt::dev_alloc(h->device, (void**)&h->status, 4 * sizeof(unsigned));
     if (e == cudaSuccess) e = cudaMemsetAsync(h->status, 0, 4 * sizeof(unsigned), h->stream);
     if (e != cudaSuccess)
     {
@@ -851,17 +947,20 @@ int lt_destroy(lt_lattice* h)
 {
     if (!h) return LT_OK;
     const lt::DeviceScope device_scope(h->device);
-    if (h->stream) cudaStreamSynchronize(h->stream);
+    // another stream may still read the buffers (an ensemble's, a copy's), and they may serve
+    // another handle at once
+    cudaDeviceSynchronize();
     void* bufs[] = { h->U,   h->U2,   h->Z,        h->P,       h->F,     h->Ubak,   h->R,      h->chainA,
                      h->Lam, h->Tloc, h->partials, h->results, h->d_aos, h->status, h->chainB, h->Xz,
                      h->tensor, h->rectD, h->rectE };
     for (void* p : bufs)
-        if (p) cudaFree(p);
-    for (void* p : h->levels) cudaFree(p);
-    for (void* p : h->staples) cudaFree(p);
+        if (p) lt::dev_free(h->device, p);
+    for (void* p : h->levels) lt::dev_free(h->device, p);
+    for (void* p : h->staples) lt::dev_free(h->device, p);
     if (h->h_results) cudaFreeHost(h->h_results);
     if (h->h_stage) cudaFreeHost(h->h_stage);
     if (h->stream) cudaStreamDestroy(h->stream);
+    lt::dev_handle_gone(h->device);
     delete h;
     return LT_OK;
 }
