@@ -131,11 +131,13 @@ public:
     virtual void clover_R(const Ctx& c, const void* U, void* R) const = 0;
     // sum over sites of ReTr(R01 R23 - R02 R13 + R03 R12) into results[slot]
     virtual void topcharge_R(const Ctx& c, const void* R, int slot) const = 0;
-    virtual void clover_deriv(const Ctx& c, const void* U, const void* R, void* out, double scale) const = 0;
-    virtual void stout_lambda(const Ctx& c, const void* U, const void* Up, const void* Sigma, void* Lam,
+    // K: scratch of corner_bytes (null: without it); Lt: an algebra field beside Lam (null: without it)
+    virtual size_t corner_bytes(const Geom& g) const = 0;
+    virtual void clover_deriv(const Ctx& c, const void* U, const void* R, void* K, void* out, double scale) const = 0;
+    virtual void stout_lambda(const Ctx& c, const void* U, const void* Up, const void* Sigma, void* Lam, void* Lt,
                               void* Tloc, double rho, const void* st_in) const = 0;
-    virtual void stout_recursion(const Ctx& c, const void* U, const void* Lam, const void* Tloc, void* Sigma,
-                                 double rho) const = 0;
+    virtual void stout_recursion(const Ctx& c, const void* U, const void* Lam, const void* Lt, const void* Tloc,
+                                 void* Sigma, double rho) const = 0;
 };
 
 const Backend* backend_fp64();

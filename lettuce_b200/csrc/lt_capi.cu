@@ -323,11 +323,16 @@ int metad_backward(lt_lattice* h, double rho, int n_stout, double dvdq, bool hav
     if (!have_R) LT_TRY(metad_clover(h, n_stout));
     const lt::Ctx c = h->ctx();
     const void* top = level(h, n_stout);
-    h->be->clover_deriv(c, top, h->R, h->F, dvdq);
+    // scratch that halves the derivative's products and, for FP32 links, takes a fifth of the recursion's
+    // (in FP64 the Lambda kernel, at its register limit, loses as much); where there is no memory both do
+    // without
+    (void)try_ensure(h, &h->corners, h->be->corner_bytes(h->g));
+    if (n_stout > 0 && h->be->real_bytes() == 4) (void)try_ensure(h, &h->Lt, h->be->alg_bytes(h->g));
+    h->be->clover_deriv(c, top, h->R, h->corners, h->F, dvdq);
     for (int k = n_stout; k > 0; --k)
     {
-        h->be->stout_lambda(c, level(h, k - 1), level(h, k), h->F, h->Lam, h->Tloc, rho, h->staples[k - 1]);
-        h->be->stout_recursion(c, level(h, k - 1), h->Lam, h->Tloc, h->F, rho);
+        h->be->stout_lambda(c, level(h, k - 1), level(h, k), h->F, h->Lam, h->Lt, h->Tloc, rho, h->staples[k - 1]);
+        h->be->stout_recursion(c, level(h, k - 1), h->Lam, h->Lt, h->Tloc, h->F, rho);
     }
     return launched("metad_backward");
 }
@@ -952,7 +957,7 @@ int lt_destroy(lt_lattice* h)
     cudaDeviceSynchronize();
     void* bufs[] = { h->U,   h->U2,   h->Z,        h->P,       h->F,     h->Ubak,   h->R,      h->chainA,
                      h->Lam, h->Tloc, h->partials, h->results, h->d_aos, h->status, h->chainB, h->Xz,
-                     h->tensor, h->rectD, h->rectE };
+                     h->tensor, h->rectD, h->rectE, h->Lt, h->corners };
     for (void* p : bufs)
         if (p) lt::dev_free(h->device, p);
     for (void* p : h->levels) lt::dev_free(h->device, p);

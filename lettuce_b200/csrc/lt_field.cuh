@@ -219,6 +219,41 @@ template <typename T> struct Alg
     }
 };
 
+// Hermitian matrices (9 reals) per site on any number of planes, plane index (plane*2 + parity)*9 + k
+template <typename T> struct HermPlanes
+{
+    T* __restrict__ p;
+    int vh;
+
+    LT_D size_t plane(int pl, int par) const { return (size_t)((pl * 2 + par) * 9) * (size_t)vh; }
+    LT_D void st(int pl, int par, int s, const M3<T>& h) const
+    {
+        T* q = p + plane(pl, par) + s;
+        const T v[9] = { h.e[0][0].r, h.e[1][1].r, h.e[2][2].r, h.e[0][1].r, h.e[0][1].i,
+                         h.e[0][2].r, h.e[0][2].i, h.e[1][2].r, h.e[1][2].i };
+#pragma unroll
+        for (int k = 0; k < 9; ++k) q[(size_t)k * vh] = v[k];
+    }
+    LT_D M3<T> ld(int pl, int par, int s) const
+    {
+        const T* q = p + plane(pl, par) + s;
+        T v[9];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) v[k] = q[(size_t)k * vh];
+        M3<T> m;
+        m.e[0][0] = mkc<T>(v[0], 0);
+        m.e[1][1] = mkc<T>(v[1], 0);
+        m.e[2][2] = mkc<T>(v[2], 0);
+        m.e[0][1] = mkc<T>(v[3], v[4]);
+        m.e[0][2] = mkc<T>(v[5], v[6]);
+        m.e[1][2] = mkc<T>(v[7], v[8]);
+        m.e[1][0] = mkc<T>(v[3], -v[4]);
+        m.e[2][0] = mkc<T>(v[5], -v[6]);
+        m.e[2][1] = mkc<T>(v[7], -v[8]);
+        return m;
+    }
+};
+
 // Full 3x3 complex per link (used for the local term of the stout-force recursion)
 template <typename T> struct Full
 {

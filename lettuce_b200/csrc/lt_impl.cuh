@@ -484,18 +484,28 @@ public:
         k_topcharge_R<T><<<kRedBlocks, kRedThreads, 0, c.stream>>>(clov(R, c.g), c.g, c.partials + (size_t)slot * kRedBlocks);
         finish(c, slot, 1);
     }
-    void clover_deriv(const Ctx& c, const void* U, const void* R, void* out, double scale) const override
+    size_t corner_bytes(const Geom& g) const override { return (size_t)12 * g.V * 9 * sizeof(T); }
+    void clover_deriv(const Ctx& c, const void* U, const void* R, void* K, void* out, double scale) const override
     {
-        launch_chained(k_clover_deriv<T, NR>, nblocks(c.g.V, kSitesPerBlock), 4 * kSitesPerBlock, c.stream,
-                       gauge(U, c.g), clov(R, c.g), alg(out, c.g), c.g, (T)scale);
+        const int nb = nblocks(c.g.V, kSitesPerBlock);
+        if (K)
+        {
+            const HermPlanes<T> k{ (T*)K, c.g.vh };
+            launch_chained(k_clover_corners<T, NR>, nb, 384, c.stream, gauge(U, c.g), clov(R, c.g), k, c.g);
+            launch_chained(k_clover_deriv_corners<T, NR>, nb, 4 * kSitesPerBlock, c.stream, gauge(U, c.g), k,
+                           alg(out, c.g), c.g, (T)scale);
+            return;
+        }
+        launch_chained(k_clover_deriv<T, NR>, nb, 4 * kSitesPerBlock, c.stream, gauge(U, c.g), clov(R, c.g),
+                       alg(out, c.g), c.g, (T)scale);
     }
-    void stout_lambda(const Ctx& c, const void* U, const void* Up, const void* Sigma, void* Lam, void* Tloc,
+    void stout_lambda(const Ctx& c, const void* U, const void* Up, const void* Sigma, void* Lam, void* Lt, void* Tloc,
                       double rho, const void* st_in) const override
     {
         if (st_in)
         {
             launch_chained(k_stout_lambda_st<T, NR>, nblocks(c.g.V, kSitesPerBlock), 4 * kSitesPerBlock, c.stream,
-                           gauge(U, c.g), gauge(Up, c.g), alg(Sigma, c.g), alg(Lam, c.g), full(Tloc, c.g),
+                           gauge(U, c.g), gauge(Up, c.g), alg(Sigma, c.g), alg(Lam, c.g), alg(Lt, c.g), full(Tloc, c.g),
                            full(st_in, c.g), c.g, (T)rho);
             return;
         }
@@ -503,18 +513,20 @@ public:
         {
             prefer_shared<k_stout_lambda_staged<0>>();
             launch_chained(k_stout_lambda_staged<0>, nblocks(c.g.V, kSitesPerBlock), 4 * kSitesPerBlock, c.stream,
-                           gauge(U, c.g), gauge(Up, c.g), alg(Sigma, c.g), alg(Lam, c.g), full(Tloc, c.g), c.g,
-                           (T)rho);
+                           gauge(U, c.g), gauge(Up, c.g), alg(Sigma, c.g), alg(Lam, c.g), alg(Lt, c.g), full(Tloc, c.g),
+                           c.g, (T)rho);
             return;
         }
         launch_chained(k_stout_lambda<T, NR>, nblocks(c.g.V, kSitesPerBlock), 4 * kSitesPerBlock, c.stream,
-                       gauge(U, c.g), gauge(Up, c.g), alg(Sigma, c.g), alg(Lam, c.g), full(Tloc, c.g), c.g, (T)rho);
+                       gauge(U, c.g), gauge(Up, c.g), alg(Sigma, c.g), alg(Lam, c.g), alg(Lt, c.g), full(Tloc, c.g), c.g,
+                       (T)rho);
     }
-    void stout_recursion(const Ctx& c, const void* U, const void* Lam, const void* Tloc, void* Sigma,
+    void stout_recursion(const Ctx& c, const void* U, const void* Lam, const void* Lt, const void* Tloc, void* Sigma,
                          double rho) const override
     {
-        launch_chained(k_stout_recursion<T, NR>, nblocks(c.g.V, kSitesPerBlock), 4 * kSitesPerBlock, c.stream,
-                       gauge(U, c.g), alg(Lam, c.g), full(Tloc, c.g), alg(Sigma, c.g), c.g, (T)rho);
+        launch_chained(Lt ? k_stout_recursion<T, NR, true> : k_stout_recursion<T, NR, false>,
+                       nblocks(c.g.V, kSitesPerBlock), 4 * kSitesPerBlock, c.stream, gauge(U, c.g), alg(Lam, c.g),
+                       alg(Lt, c.g), full(Tloc, c.g), alg(Sigma, c.g), c.g, (T)rho);
     }
 };
 

@@ -282,6 +282,33 @@ template <typename T> LT_HD M3<T> unpack_h(const A8<T>& x)
     return m;
 }
 
+// V^dag H V (UP = false) or V H V^dag (UP = true) of a Hermitian H (real diagonal) for a unitary V,
+// the full Hermitian matrix
+template <bool UP, typename T> LT_HD M3<T> conjugate_h(const M3<T>& h, const M3<T>& v)
+{
+    const M3<T> w = UP ? mul_xh(v, h) : mul_hx(h, v);
+    M3<T> r;
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = i; j < 3; ++j)
+        {
+            T re = 0, im = 0;   // UP: W_ik conj(V_jk); else conj(V_ki) W_kj
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+            {
+                const cx<T> a = UP ? w.e[i][k] : w.e[k][j], b = UP ? v.e[j][k] : v.e[k][i];
+                re += a.r * b.r;
+                re += a.i * b.i;
+                im += a.i * b.r;
+                im -= a.r * b.i;
+            }
+            r.e[i][j] = mkc<T>(re, i == j ? (T)0 : im);
+            if (i != j) r.e[j][i] = mkc<T>(re, -im);
+        }
+    return r;
+}
+
 // ---------------------------------------------------------------- reunitarisation
 // RestoreLastRow (math/su3.hpp:362-367): row 2 = conj(row 0 x row 1)
 // g1 a + g2 b as an FMA chain
