@@ -26,6 +26,7 @@ struct Ctx
     // forces over all links; null: no memory for them, the rectangles are multiplied out directly
     void* rectD = nullptr;
     void* rectE = nullptr;
+    void* planes = nullptr;       // plaquette planes of the Wilson force (plane_bytes); null: no memory for them
     unsigned* order = nullptr;    // the handle's launch counter for alternating site orders
 };
 
@@ -88,8 +89,8 @@ public:
                         uint64_t seed, int max_iter) const = 0;
     virtual void heatbath(const Ctx& c, void* U, int mu, int par, double prefactor, uint64_t counter,
                           uint64_t seed, int max_iter) const = 0;
-    // flow_split(): the format runs a flow stage as two kernels and wants an algebra scratch
-    // field X (flow_stage's last argument; null: the fused stage)
+    // flow_split(): the format runs a flow stage without planes as two kernels and wants an algebra
+    // scratch field X (flow_stage's last argument; null: the fused stage)
     virtual bool flow_split() const = 0;
     virtual void flow_stage(const Ctx& c, const void* Uin, void* Uout, void* Z, double c_old, double c_new,
                             double c_exp, int read_z, int write_z, void* X) const = 0;
@@ -103,6 +104,11 @@ public:
 
     virtual void momenta(const Ctx& c, const void* U, void* P, const void* F, double coef, double eps) const = 0;
     virtual void fields(const Ctx& c, void* U, const void* P, double eps) const = 0;
+    // momenta() then fields(eps_drift), Uin -> Uout; md_fused(): the storage and action have it
+    virtual bool md_fused(const Ctx& c) const = 0;
+    virtual void md_step(const Ctx& c, const void* Uin, void* Uout, void* P, const void* F, double coef, double eps,
+                         double eps_drift) const = 0;
+    virtual size_t plane_bytes(const Geom& g) const = 0;     // the plaquette planes; 0: the storage does not use them
     virtual void random_momenta(const Ctx& c, void* P, uint64_t counter, uint64_t seed) const = 0;
     // P <- a P + b F on algebra fields (F may be null); the spatial parity reflection Uin -> Uout
     virtual void alg_axpby(const Ctx& c, void* P, const void* F, double a, double b) const = 0;

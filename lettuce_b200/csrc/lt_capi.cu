@@ -149,10 +149,16 @@ bool try_ensure(lt_lattice* h, void** p, size_t bytes)
     return false;
 }
 
-// The scratch fields of a rectangle force over all links.  On the largest lattices there may be no
-// memory for them; the force is then multiplied out path by path, as it is without them.
-void ensure_rect(lt_lattice* h)
+// The scratch fields of a force over all links (rect: with rectangles).  On the largest lattices there may
+// be no memory for them; the staples are then multiplied out link by link, as they are without them.
+void ensure_force(lt_lattice* h, bool rect)
 {
+    if (!rect)
+    {
+        const size_t bytes = h->be->plane_bytes(h->g);
+        if (bytes) (void)try_ensure(h, &h->planes, bytes);
+        return;
+    }
     if (h->rectE) return;
     if (try_ensure(h, &h->rectD, h->be->gauge_bytes(h->g)) && try_ensure(h, &h->rectE, h->be->full_bytes(h->g))) return;
     if (h->rectD) lt::dev_free(h->device, h->rectD);
@@ -217,8 +223,9 @@ int flow_steps(lt_lattice* h, double eps, int n_step, int integrator = LT_FLOW_R
     LT_TRY(ensure(h, &h->U2, h->be->gauge_bytes(h->g)));
     if (ns > 1) LT_TRY(ensure(h, &h->Z, h->be->alg_bytes(h->g)));
     const bool zeuthen = h->flow_action == LT_FLOW_ACTION_ZEUTHEN;
-    if (zeuthen || h->be->flow_split()) LT_TRY(ensure(h, &h->Xz, h->be->alg_bytes(h->g)));
-    if (zeuthen || h->act_radius == 2) ensure_rect(h);
+    ensure_force(h, zeuthen || h->act_radius == 2);
+    const bool split = h->be->flow_split() && (h->act_radius == 2 || !h->planes);
+    if (zeuthen || split) LT_TRY(ensure(h, &h->Xz, h->be->alg_bytes(h->g)));
     const lt::Ctx c = h->ctx();
     for (int k = 0; k < n_step; ++k)
         for (int j = 0; j < ns; ++j)
@@ -230,7 +237,7 @@ int flow_steps(lt_lattice* h, double eps, int n_step, int integrator = LT_FLOW_R
                                           st[j].read_z, st[j].write_z, 5.0 / 3.0, -1.0 / 12.0);
             else
                 h->be->flow_stage(c, h->U, h->U2, h->Z, st[j].c_old, st[j].c_new * eps, st[j].c_exp, st[j].read_z,
-                                  st[j].write_z, h->be->flow_split() ? h->Xz : nullptr);
+                                  st[j].write_z, split ? h->Xz : nullptr);
             std::swap(h->U, h->U2);
         }
     return launched("flow");
@@ -383,7 +390,9 @@ int metad_force_now(lt_lattice* h, const MetaDParams* md, bool submeasure)
     return metad_backward(h, md->rho, md->n_stout, md->bias->derivative(q), true);
 }
 
-int kick(lt_lattice* h, double beta, double eps, const MetaDParams* md, bool submeasure)
+// With drift_eps set, the drift of that length follows in the same kernel.
+int kick(lt_lattice* h, double beta, double eps, const MetaDParams* md, bool submeasure,
+         const double* drift_eps = nullptr)
 {
     const void* F = nullptr;
     if (md)
@@ -391,7 +400,12 @@ int kick(lt_lattice* h, double beta, double eps, const MetaDParams* md, bool sub
         LT_TRY(metad_force_now(h, md, submeasure));
         F = h->F;
     }
-    if (h->act_radius == 2) ensure_rect(h);
+    if (drift_eps)
+    {
+        h->be->md_step(h->ctx(), h->U, h->U2, h->P, F, beta / 6.0, eps, *drift_eps);
+        std::swap(h->U, h->U2);
+        return launched("md_step");
+    }
     h->be->momenta(h->ctx(), h->U, h->P, F, beta / 6.0, eps);
     return launched("momenta");
 }
@@ -556,13 +570,22 @@ int md_check(int integ, bool metad, const char* fn)
 // Run a program on (h->U, h->P); md null for the gauge action alone
 int integrate(lt_lattice* h, double beta, const std::vector<MdOp>& ops, const MetaDParams* md)
 {
+    ensure_force(h, h->act_radius == 2);
     const lt::Ctx c = h->ctx();
-    for (const MdOp& op : ops)
+    // a kick and the drift after it run together where the storage and the action have that and
+    // there is memory for the second link field
+    const bool fused = h->be->md_fused(c) && try_ensure(h, &h->U2, h->be->gauge_bytes(h->g));
+    for (size_t k = 0; k < ops.size(); ++k)
     {
+        const MdOp& op = ops[k];
+        const double* drift_eps = nullptr;
+        if (fused && (op.kind == Md::KICK || op.kind == Md::KICK_GAUGE) && k + 1 < ops.size() &&
+            ops[k + 1].kind == Md::DRIFT)
+            drift_eps = &ops[++k].eps;
         switch (op.kind)
         {
-        case Md::KICK: LT_TRY(kick(h, beta, op.eps, md, op.sub)); break;
-        case Md::KICK_GAUGE: LT_TRY(kick(h, beta, op.eps, nullptr, false)); break;
+        case Md::KICK: LT_TRY(kick(h, beta, op.eps, md, op.sub, drift_eps)); break;
+        case Md::KICK_GAUGE: LT_TRY(kick(h, beta, op.eps, nullptr, false, drift_eps)); break;
         case Md::KICK_METAD:
             LT_TRY(metad_force_now(h, md, op.sub));
             h->be->alg_axpby(c, h->P, h->F, 1.0, op.eps);
@@ -957,7 +980,7 @@ int lt_destroy(lt_lattice* h)
     cudaDeviceSynchronize();
     void* bufs[] = { h->U,   h->U2,   h->Z,        h->P,       h->F,     h->Ubak,   h->R,      h->chainA,
                      h->Lam, h->Tloc, h->partials, h->results, h->d_aos, h->status, h->chainB, h->Xz,
-                     h->tensor, h->rectD, h->rectE, h->Lt, h->corners };
+                     h->tensor, h->rectD, h->rectE, h->planes, h->Lt, h->corners };
     for (void* p : bufs)
         if (p) lt::dev_free(h->device, p);
     for (void* p : h->levels) lt::dev_free(h->device, p);
@@ -1673,7 +1696,7 @@ int lt_gauge_force(lt_lattice* h, double beta, double* force_out)
     if (!force_out) return lt::set_error(LT_ERR_ARG, "lt_gauge_force: null pointer");
     LT_TRY(ensure(h, &h->F, h->be->alg_bytes(h->g)));
     LT_CK(cudaMemsetAsync(h->F, 0, h->be->alg_bytes(h->g), h->stream));
-    if (h->act_radius == 2) ensure_rect(h);
+    ensure_force(h, h->act_radius == 2);
     h->be->momenta(h->ctx(), h->U, h->F, nullptr, beta / 6.0, 1.0);
     LT_TRY(ensure_aos(h));
     h->be->alg_to_aos(h->ctx(), h->F, h->d_aos);

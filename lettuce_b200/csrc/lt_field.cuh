@@ -254,6 +254,43 @@ template <typename T> struct HermPlanes
     }
 };
 
+// One algebra element (A8) per site and plane mu < nu (planes 01 02 03 12 13 23), in 16-byte chunks:
+// chunk c of (plane, parity) at ((plane * 2 + parity) * NC + c) * vh, NC = 2 (FP32) or 4 (FP64)
+template <typename T> struct PlaneAlg
+{
+    static constexpr int NC = (int)sizeof(T) / 2, W = 16 / (int)sizeof(T);
+    struct __align__(16) Chunk { T v[W]; };
+    Chunk* __restrict__ p;
+    int vh;
+
+    LT_D size_t at(int pl, int par, int s) const { return (size_t)(pl * 2 + par) * NC * (size_t)vh + s; }
+    LT_D A8<T> ld(int pl, int par, int s) const
+    {
+        A8<T> x;
+        const Chunk* q = p + at(pl, par, s);
+#pragma unroll
+        for (int c = 0; c < NC; ++c)
+        {
+            const Chunk k = q[(size_t)c * vh];
+#pragma unroll
+            for (int w = 0; w < W; ++w) x.a[c * W + w] = k.v[w];
+        }
+        return x;
+    }
+    LT_D void st(int pl, int par, int s, const A8<T>& x) const
+    {
+        Chunk* q = p + at(pl, par, s);
+#pragma unroll
+        for (int c = 0; c < NC; ++c)
+        {
+            Chunk k;
+#pragma unroll
+            for (int w = 0; w < W; ++w) k.v[w] = x.a[c * W + w];
+            q[(size_t)c * vh] = k;
+        }
+    }
+};
+
 // Full 3x3 complex per link (used for the local term of the stout-force recursion)
 template <typename T> struct Full
 {

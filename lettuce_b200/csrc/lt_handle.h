@@ -95,6 +95,7 @@ struct lt_lattice
     // force of the gradient flow run into this handle (lt_set_flow_action): the gauge action's
     // (LT_FLOW_ACTION_GAUGE, the reference's GradientFlowKernel) or the Zeuthen flow's
     int flow_action = LT_FLOW_ACTION_GAUGE;
+    void* planes = nullptr;      // plaquette planes of the Wilson force
     void* rectD = nullptr;       // two-link products of the rectangle forces (link field)
     void* rectE = nullptr;       // and their outer staples (full matrices)
     void* Xz = nullptr;          // Luescher-Weisz force of a Zeuthen flow stage (algebra)
@@ -112,6 +113,7 @@ struct lt_lattice
         c.rect = act_radius == 2;
         c.cp = act_cp;
         c.cr = act_cr;
+        c.planes = planes;
         c.rectD = rectD;
         c.rectE = rectE;
         c.order = &order;

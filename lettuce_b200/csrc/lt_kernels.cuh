@@ -1841,6 +1841,117 @@ __global__ void __launch_bounds__(4 * kSitesPerBlock, LT_MINB_FLOW_STAGED)
     Uout.st(mu, par, s, exp_update<float, 2>(unpack_ah(z), c_exp, u));
 }
 
+// ---------------------------------------------------------------- plaquette forces
+// The Wilson force of all links from the plaquettes' algebra elements, on the 18-real storages.  With
+// F_{mu nu}(x) = Algebra(P_{mu nu}(x)), P the plaquette that starts at x along mu,
+//   Algebra(st U_mu(x)^dag) = sum_{nu != mu} [U_nu(x-nu)^dag F_{mu nu}(x-nu) U_nu(x-nu) - F_{mu nu}(x)]:
+// the upper staples close to P_{nu mu}(x) = P_{mu nu}(x)^dag, the lower ones to the plaquette at x - nu
+// carried along the link between them.  Every plaquette is multiplied out once for its four links
+// instead of once for each: 870 multiply-adds a link for the force against 1,390 from the staple, and
+// 8 link loads against 19, at far fewer registers (FP64: 140 and 160 in the two kernels, 255 in the
+// staple's).  Bound by issue and HBM together (the planes cross it once each way).  An RK3 stage, before and
+// now: FP64 32^4 1129 and 923 us, 16^4 65 and 51; FP32 32^4 611 and 491, 16^4 33 and 27; a kick and its
+// drift FP64 32^4 1050 and 941, FP32 606 and 501.  Working through slabs of timeslices, so that the planes
+// stay in L2, was slower (FP64 32^4 953 to 1004 us): more launches and tails than traffic saved.  Two-row links
+// keep the staged staple: 5 % less for the planes, but a third row rebuilt at both ends of every conjugation
+// costs them accuracy in the charge of a long flow (2.6e-5 at t = 1 on the 32^4 fixture, 7e-6 staged).
+template <typename T>
+__global__ void __launch_bounds__(192) k_plaq_planes(Gauge<T, 3> U, PlaneAlg<T> F, Geom g, int rev)
+{
+    pdl_release();
+    pdl_wait();
+    const int pl = threadIdx.x >> 5;   // warp = plane, lanes = consecutive sites
+    int x = blockIdx.x * kSitesPerBlock + (threadIdx.x & 31);
+    if (x >= g.V) return;
+    if (rev) x = g.V - 1 - x;
+    const int par = x >= g.vh, s = x - par * g.vh, op = par ^ 1;
+    int c[4];
+    const int i = site_coords(g, par, s, c);
+    const int a = pl < 3 ? 0 : pl < 5 ? 1 : 2, b = pl < 3 ? pl + 1 : pl < 5 ? pl - 1 : 3;
+    const int sa = (i + step_up_rt(g, a, c)) >> 1, sb = (i + step_up_rt(g, b, c)) >> 1;
+    // P = (U_a(x) U_b(x+a)) (U_b(x) U_a(x+b))^dag
+    const M3<T> A = mul(U.ld(a, par, s), U.ld(b, op, sa));
+    const M3<T> B = mul(U.ld(b, par, s), U.ld(a, op, sb));
+    F.st(pl, par, s, algebra8_nd(A, B));
+}
+
+// Algebra(st U^dag) of the link (mu, x) from the planes
+template <typename T>
+LT_D A8<T> plane_force(const Gauge<T, 3>& U, const PlaneAlg<T>& F, const Geom& g, int par, int i, const int c[4], int mu)
+{
+    A8<T> a;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) a.a[k] = 0;
+#pragma unroll
+    for (int n = 0; n < 3; ++n)
+    {
+        const int nu = n + (n >= mu ? 1 : 0), lo = mu < nu ? mu : nu, hi = mu < nu ? nu : mu;
+        const int pl = lo == 0 ? hi - 1 : lo == 1 ? hi + 1 : 5;
+        const T sign = mu < nu ? (T)1 : (T)-1;
+        const int sd = (i + step_dn_rt(g, nu, c)) >> 1;
+        const A8<T> up = F.ld(pl, par, i >> 1);
+        const A8<T> dn = transport8(F.ld(pl, par ^ 1, sd), U.ld(nu, par ^ 1, sd));
+#pragma unroll
+        for (int k = 0; k < 8; ++k) a.a[k] += sign * (dn.a[k] - up.a[k]);
+    }
+    return a;
+}
+
+// What a link does with its force a = Algebra(st U^dag):
+//   Flow   Z <- c_old Z + c_new a, U' = exp(c_exp Z) U       (a stage of a flow integrator)
+//   Kick   P <- P + c_new (c_old a + F)                      (UpdateMomenta, c_old = beta / 6)
+//   Md     Kick, then U' = exp(c_exp P) U                    (UpdateMomenta and the UpdateFields after it)
+enum class Step { Flow, Kick, Md };
+// 6 blocks of 128 per SM for FP32 (491 us for a 32^4 stage, 512 with 5), 3 for FP64 (160 registers, nothing
+// spilled)
+template <typename T, Step STEP>
+__global__ void __launch_bounds__(kThreads, sizeof(T) == 4 ? 6 : 3)
+    k_plane_step(Gauge<T, 3> Uin, Gauge<T, 3> Uout, PlaneAlg<T> F, Alg<T> Z, Alg<T> X, Geom g, T c_old, T c_new, T c_exp,
+                 int read, int write, int rev)
+{
+    pdl_release();
+    pdl_wait();
+    int mu, x;
+    if (!link_of_thread(g, mu, x, rev)) return;
+    const int par = x >= g.vh, s = x - par * g.vh;
+    int c[4];
+    const int i = site_coords(g, par, s, c);
+    const A8<T> a = plane_force(Uin, F, g, par, i, c, mu);
+    A8<T> z;
+    if (STEP == Step::Flow)
+    {
+        if (read)
+        {
+            const A8<T> zo = Z.ld(mu, par, s);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) z.a[k] = c_old * zo.a[k] + c_new * a.a[k];
+        }
+        else
+        {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) z.a[k] = c_new * a.a[k];
+        }
+        if (write) Z.st(mu, par, s, z);
+    }
+    else
+    {
+        z = Z.ld(mu, par, s);
+        if (read)   // F of the smeared charge
+        {
+            const A8<T> f = X.ld(mu, par, s);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) z.a[k] += c_new * (c_old * a.a[k] + f.a[k]);
+        }
+        else
+        {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) z.a[k] += c_new * c_old * a.a[k];
+        }
+        Z.st(mu, par, s, z);
+    }
+    if (STEP != Step::Kick) Uout.st(mu, par, s, exp_update<T, 3>(unpack_ah(z), c_exp, Uin.ld(mu, par, s)));
+}
+
 // ---------------------------------------------------------------- Zeuthen flow
 // The Zeuthen flow (Ramos and Sint, Eur. Phys. J. C 76 (2016) 15, arXiv:1508.05552; not in the
 // reference, which flows with the simulated action's force only, gradient_flow.hpp:298-332):
@@ -2460,6 +2571,39 @@ __global__ void __launch_bounds__(4 * kSitesPerBlock, LT_MINB_FLOW_STAGED)
 #pragma unroll
     for (int k = 0; k < 8; ++k) p.a[k] += use_f ? eps * (coef * a.a[k] + f.a[k]) : eps * coef * a.a[k];
     P.st(mu, par, s, p);
+}
+
+// A kick and the drift that follows it (UpdateMomenta then UpdateFields) for every link, on two-row FP32
+// storage with the staged staple (ACT: Wilson or TwoLink):
+//   P <- P + eps (beta/6 Algebra(st U^dag) + F),  U' = exp(eps_drift P) U, Gram-Schmidt,
+// Uin -> Uout as a flow stage, so that all staples see the field before the drift.  The drift alone reads the
+// link and the momenta again that the kick has in registers: 463 us for the two kernels at 32^4, 415 fused.
+// F is read after the staple (held through it, it would cost the kernel its fifth block per SM).
+template <Act ACT>
+__global__ void __launch_bounds__(4 * kSitesPerBlock, LT_MINB_FLOW_STAGED)
+    k_md_step_staged(Gauge<float, 2> Uin, Gauge<float, 2> Uout, Alg<float> P, Alg<float> F, Geom g, float coef, float eps,
+                     float eps_drift, int use_f, RectFields<float, 2> W, float cp, float cr, int rev)
+{
+    __shared__ StapleRing ring;
+    pdl_release();
+    pdl_wait();
+    int mu, x;
+    if (!link_of_thread(g, mu, x, rev)) return;
+    const int par = x >= g.vh, s = x - par * g.vh;
+    int c[4];
+    const int i = site_coords(g, par, s, c);
+    A8<float> p = P.ld(mu, par, s);
+    M3<float> u;
+    const M3<float> st = ACT == Act::TwoLink ? staple_two_link_staged(ring, Uin, W, g, par, i, s, c, mu, cp, cr, u)
+                                             : staple_staged<true>(ring, Uin, g, par, i, s, c, mu, u);
+    const A8<float> a = algebra8(mul_nd(st, u));
+    A8<float> f;
+    if (use_f)
+        f = F.ld(mu, par, s);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) p.a[k] += use_f ? eps * (coef * a.a[k] + f.a[k]) : eps * coef * a.a[k];
+    P.st(mu, par, s, p);
+    Uout.st(mu, par, s, exp_update<float, 2>(unpack_ah(p), eps_drift, u));
 }
 
 // U <- exp(eps P) U, Gram-Schmidt (updates/hmc_gauge.hpp:505-523)

@@ -249,6 +249,94 @@ template <typename T> LT_HD M3<T> unpack_ah(const A8<T>& x)
     return m;
 }
 
+// Algebra(A B^dag), packed, without forming the product
+template <typename T> LT_HD A8<T> algebra8_nd(const M3<T>& a, const M3<T>& b)
+{
+    T d[3];
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+    {
+        d[i] = 0;
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+        {
+            d[i] += a.e[i][k].i * b.e[i][k].r;
+            d[i] -= a.e[i][k].r * b.e[i][k].i;
+        }
+    }
+    A8<T> x;
+    const T t = (d[0] + d[1] + d[2]) * (T)(1.0 / 3.0);
+    x.a[0] = d[0] - t;
+    x.a[1] = d[1] - t;
+#pragma unroll
+    for (int o = 0; o < 3; ++o)
+    {
+        const int i = o == 2 ? 1 : 0, j = o == 0 ? 1 : 2;
+        T re = 0, im = 0;   // (A B^dag)_ij - conj((A B^dag)_ji)
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+        {
+            re += a.e[i][k].r * b.e[j][k].r;
+            re += a.e[i][k].i * b.e[j][k].i;
+            re -= a.e[j][k].r * b.e[i][k].r;
+            re -= a.e[j][k].i * b.e[i][k].i;
+            im += a.e[i][k].i * b.e[j][k].r;
+            im -= a.e[i][k].r * b.e[j][k].i;
+            im += a.e[j][k].i * b.e[i][k].r;
+            im -= a.e[j][k].r * b.e[i][k].i;
+        }
+        x.a[2 + 2 * o] = (T)0.5 * re;
+        x.a[3 + 2 * o] = (T)0.5 * im;
+    }
+    return x;
+}
+
+// V^dag X V of a traceless anti-Hermitian X for a unitary V, packed (X = i H, H Hermitian)
+template <typename T> LT_HD A8<T> transport8(const A8<T>& x, const M3<T>& v)
+{
+    M3<T> h;
+    h.e[0][0] = mkc<T>(x.a[0], 0);
+    h.e[1][1] = mkc<T>(x.a[1], 0);
+    h.e[2][2] = mkc<T>(-(x.a[0] + x.a[1]), 0);
+    h.e[0][1] = mkc<T>(x.a[3], -x.a[2]);
+    h.e[0][2] = mkc<T>(x.a[5], -x.a[4]);
+    h.e[1][2] = mkc<T>(x.a[7], -x.a[6]);
+    h.e[1][0] = mkc<T>(x.a[3], x.a[2]);
+    h.e[2][0] = mkc<T>(x.a[5], x.a[4]);
+    h.e[2][1] = mkc<T>(x.a[7], x.a[6]);
+    const M3<T> w = mul_hx(h, v);
+    A8<T> y;
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+    {
+        T d = 0;
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+        {
+            d += v.e[k][i].r * w.e[k][i].r;
+            d += v.e[k][i].i * w.e[k][i].i;
+        }
+        y.a[i] = d;
+    }
+#pragma unroll
+    for (int o = 0; o < 3; ++o)
+    {
+        const int i = o == 2 ? 1 : 0, j = o == 0 ? 1 : 2;
+        T re = 0, im = 0;   // conj(V_ki) W_kj
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+        {
+            re += v.e[k][i].r * w.e[k][j].r;
+            re += v.e[k][i].i * w.e[k][j].i;
+            im += v.e[k][i].r * w.e[k][j].i;
+            im -= v.e[k][i].i * w.e[k][j].r;
+        }
+        y.a[2 + 2 * o] = -im;
+        y.a[3 + 2 * o] = re;
+    }
+    return y;
+}
+
 // Hermitian traceless H kept as 8 reals: H00 = h0, H11 = h1, H22 = -(h0+h1), H01 = h2 + i h3, ...
 // TracelessHermitian(M) = (M + M^dag)/2 - tr(M + M^dag)/6 (math/su3.hpp:445-448), packed
 template <typename T> LT_HD A8<T> traceless_herm8(const M3<T>& m)

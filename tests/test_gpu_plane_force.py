@@ -1,0 +1,40 @@
+"""The Wilson force from the plaquette planes (k_plaq_planes, k_plane_step) in the three storages, as
+a force, as fused kicks and drifts and as flow stages, on lattices with partly empty blocks
+(V = 16, 96, 288, 720 sites against 32 a block) and extents of 2, against the FP64 oracle on the links as
+they are stored.
+
+Bounds: FP64 1e-12.  FP32: a plaquette entry is three products of unit rows, each a sum of three
+complex products rounded by at most 6 eps, the conjugation two more; six of them add up to at most
+6 * 5 * 6 eps = 1.1e-5 absolute, on a force whose largest entries are of order one; a step moves a
+link by at most the step size times that.
+"""
+import numpy as np
+import pytest
+
+import lettuce_b200 as lt
+from ltref import haar_links_numpy, rel_err
+
+pytestmark = pytest.mark.gpu
+
+EXTS = [(2, 2, 2, 2), (2, 4, 6, 2), (4, 6, 2, 6), (6, 2, 10, 6)]
+TOL = {"fp64": 1e-12, "fp32": 1.1e-5, "fp32_12": 1.1e-5}
+
+
+@pytest.mark.parametrize("prec", ["fp64", "fp32", "fp32_12"])
+@pytest.mark.parametrize("ext", EXTS)
+def test_force_flow_and_md(oracle, ext, prec):
+    G = lt.GaugeField(ext, prec)
+    G.upload(oracle.heatbath(ext, haar_links_numpy(ext, 5), 5.8, 2, 7, 0))
+    W = G.download()
+    want = oracle.gauge_force(ext, W, 6.0)
+    assert np.abs(lt.WilsonAction(6.0).Force(G) - want).max() < TOL[prec] * max(1.0, np.abs(want).max())
+    F = lt.GaugeField(ext, prec)
+    lt.GradientFlowKernel(G, F, lt.RK3, None, 0.02)(2)
+    assert rel_err(F.download(), oracle.flow_rk3(ext, W, 0.02, 2)) < TOL[prec]
+    k = lt.HMCKernel(G, lt.WilsonAction(6.0), 0.3, integrator=lt.OMF_2)
+    k.RandomMomentum(1)
+    P = k.GetMomenta()
+    k.Integrate(3)
+    Uo, Po = oracle.omf2(ext, W, P, 6.0, 0.3, 3)[:2]
+    assert rel_err(G.download(), Uo) < TOL[prec]
+    assert np.abs(k.GetMomenta() - Po).max() < 10.0 * TOL[prec]
