@@ -330,12 +330,16 @@ int metad_backward(lt_lattice* h, double rho, int n_stout, double dvdq, bool hav
     if (!have_R) LT_TRY(metad_clover(h, n_stout));
     const lt::Ctx c = h->ctx();
     const void* top = level(h, n_stout);
-    // scratch that halves the derivative's products and, for FP32 links, takes a fifth of the recursion's
-    // (in FP64 the Lambda kernel, at its register limit, loses as much); where there is no memory both do
-    // without
-    (void)try_ensure(h, &h->corners, h->be->corner_bytes(h->g));
-    if (n_stout > 0 && h->be->real_bytes() == 4) (void)try_ensure(h, &h->Lt, h->be->alg_bytes(h->g));
-    h->be->clover_deriv(c, top, h->R, h->corners, h->F, dvdq);
+    // scratch that halves the derivative's products on smeared links and, for FP32 links, takes a fifth of the
+    // recursion's (in FP64 the Lambda kernel, at its register limit, loses as much); where there is no memory
+    // both do without.  The links as given (no smearing) keep the direct products: the corner sums take
+    // links for unitary, as every smeared level is.
+    if (n_stout > 0)
+    {
+        (void)try_ensure(h, &h->corners, h->be->corner_bytes(h->g));
+        if (h->be->real_bytes() == 4) (void)try_ensure(h, &h->Lt, h->be->alg_bytes(h->g));
+    }
+    h->be->clover_deriv(c, top, h->R, n_stout > 0 ? h->corners : nullptr, h->F, dvdq);
     for (int k = n_stout; k > 0; --k)
     {
         h->be->stout_lambda(c, level(h, k - 1), level(h, k), h->F, h->Lam, h->Lt, h->Tloc, rho, h->staples[k - 1]);
@@ -1696,8 +1700,12 @@ int lt_gauge_force(lt_lattice* h, double beta, double* force_out)
     if (!force_out) return lt::set_error(LT_ERR_ARG, "lt_gauge_force: null pointer");
     LT_TRY(ensure(h, &h->F, h->be->alg_bytes(h->g)));
     LT_CK(cudaMemsetAsync(h->F, 0, h->be->alg_bytes(h->g), h->stream));
-    ensure_force(h, h->act_radius == 2);
-    h->be->momenta(h->ctx(), h->U, h->F, nullptr, beta / 6.0, 1.0);
+    if (h->act_radius == 2) ensure_force(h, true);
+    // the force of the links as they are given: the planes' lower staples take them for unitary, which links
+    // read from a file of FP32 accuracy are not to FP64
+    lt::Ctx c = h->ctx();
+    c.planes = nullptr;
+    h->be->momenta(c, h->U, h->F, nullptr, beta / 6.0, 1.0);
     LT_TRY(ensure_aos(h));
     h->be->alg_to_aos(h->ctx(), h->F, h->d_aos);
     LT_TRY(launched("lt_gauge_force"));

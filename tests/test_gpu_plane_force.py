@@ -38,3 +38,15 @@ def test_force_flow_and_md(oracle, ext, prec):
     Uo, Po = oracle.omf2(ext, W, P, 6.0, 0.3, 3)[:2]
     assert rel_err(G.download(), Uo) < TOL[prec]
     assert np.abs(k.GetMomenta() - Po).max() < 10.0 * TOL[prec]
+
+
+def test_given_links_of_fp32_accuracy(oracle):
+    """An FP64 handle with links rounded to FP32 (unitary to 1e-7 only): the force and the clover derivative
+    of the links as given, to FP64 rounding."""
+    ext = (4, 6, 2, 6)
+    U = oracle.heatbath(ext, haar_links_numpy(ext, 5), 5.8, 2, 7, 0).astype(np.float32).astype(np.float64)
+    G = lt.GaugeField(ext)
+    G.upload(U)
+    assert rel_err(lt.WilsonAction(6.0).Force(G), oracle.gauge_force(ext, U, 6.0)) < 1e-12
+    assert rel_err(lt.CloverDerivative(G), oracle.clover_derivative(ext, U)) < 1e-12
+    assert lt.TopChargeClover(G) == pytest.approx(oracle.topcharge(ext, U), rel=1e-11, abs=1e-13)
