@@ -979,9 +979,9 @@ int lt_destroy(lt_lattice* h)
 {
     if (!h) return LT_OK;
     const lt::DeviceScope device_scope(h->device);
-    // another stream may still read the buffers (an ensemble's, a copy's), and they may serve
-    // another handle at once
-    cudaDeviceSynchronize();
+    // the buffers may serve another handle at once: every use of them on another stream is ordered before
+    // this one (ensembles join back, copies and swaps wait)
+    if (h->stream) cudaStreamSynchronize(h->stream);
     void* bufs[] = { h->U,   h->U2,   h->Z,        h->P,       h->F,     h->Ubak,   h->R,      h->chainA,
                      h->Lam, h->Tloc, h->partials, h->results, h->d_aos, h->status, h->chainB, h->Xz,
                      h->tensor, h->rectD, h->rectE, h->planes, h->Lt, h->corners };
