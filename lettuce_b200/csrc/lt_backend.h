@@ -55,7 +55,9 @@ public:
 
     // reductions write ctx.results[slot] (and slot+1 for clover_obs: q then e)
     virtual void plaquette(const Ctx& c, const void* U, int slot) const = 0;
-    virtual void clover_obs(const Ctx& c, const void* U, int slot) const = 0;
+    // q into slot, e into slot + 1 and, with plaq set, the plaquette sum into slot + 2
+    virtual void clover_obs(const Ctx& c, const void* U, int slot, bool plaq) const = 0;
+    virtual void plaq_charge(const Ctx& c, const void* U, int slot) const = 0;
     virtual void kinetic(const Ctx& c, const void* P, int slot) const = 0;
 
     // link health: sets kStatusNonFinite / kStatusUnitarity (tolerance tol) in c.status and
@@ -63,8 +65,8 @@ public:
     virtual void check_links(const Ctx& c, const void* U, double tol, unsigned* maxbits) const = 0;
 
     // measurement bundle (SU3_main.cpp:89-235): clover densities per timeslice into partials
-    // (q then e, nbx blocks per timeslice); plaquette, rectangle and plaquette-charge sums into
-    // results[slot..slot+2]; Polyakov loop re, im into results[slot..slot+1]; straight-line
+    // (q then e, nbx blocks per timeslice); plaquette and rectangle sums into
+    // results[slot..slot+1]; Polyakov loop re, im into results[slot..slot+1]; straight-line
     // products of the links (full FP64 matrices) for square Wilson loops
     virtual void clover_timeslices(const Ctx& c, const void* U, double* partials, int nbx) const = 0;
     virtual void loops(const Ctx& c, const void* U, int slot) const = 0;

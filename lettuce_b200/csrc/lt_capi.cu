@@ -255,11 +255,12 @@ int stout_steps(lt_lattice* h, double rho, int n)
     return launched("stout");
 }
 
-int clover_q_e(lt_lattice* h, const void* U, double* q, double* e)
+int clover_q_e(lt_lattice* h, const void* U, double* q, double* e, double* plaq = nullptr)
 {
-    h->be->clover_obs(h->ctx(), U, 2);
-    double r[2];
-    LT_TRY(fetch(h, 2, 2, r));
+    h->be->clover_obs(h->ctx(), U, 2, plaq != nullptr);
+    double r[3];
+    LT_TRY(fetch(h, 2, plaq ? 3 : 2, r));
+    if (plaq) *plaq = r[2];
     if (q) *q = -1.0 / (64.0 * 4.0 * kPi * kPi) * r[0];
     if (e) *e = r[1] / (double)h->g.V;
     return LT_OK;
@@ -357,8 +358,8 @@ int hamiltonian(lt_lattice* h, double beta, double* out)
     {
         h->be->loops(c, h->U, 4);
         h->be->kinetic(c, h->P, 1);
-        double r[3], k;
-        LT_TRY(fetch(h, 4, 3, r));
+        double r[2], k;
+        LT_TRY(fetch(h, 4, 2, r));
         LT_TRY(fetch(h, 1, 1, &k));
         *out = beta * (h->act_cp * (6.0 * V - r[0] / 3.0) + h->act_cr * (12.0 * V - r[1] / 3.0)) + k;
         return LT_OK;
@@ -1256,7 +1257,7 @@ int lt_clover_timeslices(lt_lattice* h, double* q_t, double* e_t)
     const lt::DeviceScope device_scope(h->device);
     if (!q_t && !e_t) return lt::set_error(LT_ERR_ARG, "lt_clover_timeslices: null pointers");
     const int nt = h->g.n[0];
-    const int nbx = std::max(1, std::min(lt::kRedBlocks / nt, (h->g.V / nt + lt::kRedThreads - 1) / lt::kRedThreads));
+    const int nbx = std::max(1, std::min(lt::kRedBlocks / nt, (h->g.V / nt + 31) / 32));
     if (2 * nt * nbx > lt::kNumSlots * lt::kRedBlocks)
         return lt::set_error(LT_ERR_ARG, "lt_clover_timeslices: more timeslices than the partial-sum buffer holds");
     h->be->clover_timeslices(h->ctx(), h->U, h->partials, nbx);
@@ -1288,10 +1289,10 @@ int lt_topcharge_plaquette(lt_lattice* h, double* out)
     LT_TRY(check_h(h, "lt_topcharge_plaquette"));
     const lt::DeviceScope device_scope(h->device);
     if (!out) return lt::set_error(LT_ERR_ARG, "lt_topcharge_plaquette: null pointer");
-    h->be->loops(h->ctx(), h->U, 4);
-    double r[3];
-    LT_TRY(fetch(h, 4, 3, r));
-    *out = 1.0 / (16.0 * kPi * kPi) * r[2];
+    h->be->plaq_charge(h->ctx(), h->U, 4);
+    double r;
+    LT_TRY(fetch(h, 4, 1, &r));
+    *out = 1.0 / (16.0 * kPi * kPi) * r;
     return LT_OK;
 }
 
@@ -1301,8 +1302,8 @@ int lt_rect_action(lt_lattice* h, double beta, double c_plaq, double c_rect, dou
     const lt::DeviceScope device_scope(h->device);
     if (!out) return lt::set_error(LT_ERR_ARG, "lt_rect_action: null pointer");
     h->be->loops(h->ctx(), h->U, 4);
-    double r[3];
-    LT_TRY(fetch(h, 4, 3, r));
+    double r[2];
+    LT_TRY(fetch(h, 4, 2, r));
     const double V = (double)h->g.V;
     *out = beta * (c_plaq * (6.0 * V - r[0] / 3.0) + c_rect * (12.0 * V - r[1] / 3.0));
     return LT_OK;
@@ -1648,9 +1649,11 @@ int lt_flow_rk3_measure(lt_lattice* in, lt_lattice* out, double eps, int n_meas,
     for (int m = 0; m < n_meas; ++m)
     {
         LT_TRY(flow_steps(out, eps, every));
-        if (plaq_out) LT_TRY(plaq_of(out, out->U, &plaq_out[m]));
         if (q_out || e_out)
-            LT_TRY(clover_q_e(out, out->U, q_out ? &q_out[m] : nullptr, e_out ? &e_out[m] : nullptr));
+            LT_TRY(clover_q_e(out, out->U, q_out ? &q_out[m] : nullptr, e_out ? &e_out[m] : nullptr,
+                              plaq_out ? &plaq_out[m] : nullptr));
+        else if (plaq_out)
+            LT_TRY(plaq_of(out, out->U, &plaq_out[m]));
     }
     return LT_OK;
 }

@@ -160,11 +160,22 @@ public:
                                                                       c.partials + (size_t)slot * kRedBlocks);
         finish(c, slot, 1);
     }
-    void clover_obs(const Ctx& c, const void* U, int slot) const override
+    static constexpr int kCloverSiteMin = 65536;   // two-row links: sites from which one thread takes a site
+    void clover_obs(const Ctx& c, const void* U, int slot, bool plaq) const override
     {
-        k_clover_obs<T, NR><<<kRedBlocks, kRedThreads, 0, c.stream>>>(gauge(U, c.g), c.g,
-                                                                       c.partials + (size_t)slot * kRedBlocks);
-        finish(c, slot, 2);
+        if constexpr (NR == 2)
+        {
+            if (!plaq && c.g.V >= kCloverSiteMin)
+            {
+                k_clover_site<T, NR><<<kRedBlocks, kRedThreads, 0, c.stream>>>(gauge(U, c.g), c.g,
+                                                                               c.partials + (size_t)slot * kRedBlocks);
+                finish(c, slot, 2);
+                return;
+            }
+        }
+        auto k = plaq ? k_clover_obs<T, NR, true> : k_clover_obs<T, NR, false>;
+        k<<<kRedBlocks, 192, 0, c.stream>>>(gauge(U, c.g), c.g, c.partials + (size_t)slot * kRedBlocks);
+        finish(c, slot, plaq ? 3 : 2);
     }
     void kinetic(const Ctx& c, const void* P, int slot) const override
     {
@@ -233,12 +244,25 @@ public:
     }
     void clover_timeslices(const Ctx& c, const void* U, double* partials, int nbx) const override
     {
-        k_clover_timeslice<T, NR><<<dim3(nbx, c.g.n[0]), kRedThreads, 0, c.stream>>>(gauge(U, c.g), c.g, partials);
+        if constexpr (NR == 2)
+        {
+            if (c.g.V >= kCloverSiteMin)
+            {
+                k_clover_timeslice<T, NR><<<dim3(nbx, c.g.n[0]), kRedThreads, 0, c.stream>>>(gauge(U, c.g), c.g, partials);
+                return;
+            }
+        }
+        k_clover_obs<T, NR, false><<<dim3(nbx, c.g.n[0]), 192, 0, c.stream>>>(gauge(U, c.g), c.g, partials);
     }
     void loops(const Ctx& c, const void* U, int slot) const override
     {
         k_loops<T, NR><<<kRedBlocks, kRedThreads, 0, c.stream>>>(gauge(U, c.g), c.g, c.partials + (size_t)slot * kRedBlocks);
-        finish(c, slot, 3);
+        finish(c, slot, 2);
+    }
+    void plaq_charge(const Ctx& c, const void* U, int slot) const override
+    {
+        k_plaq_charge<T, NR><<<kRedBlocks, 192, 0, c.stream>>>(gauge(U, c.g), c.g, c.partials + (size_t)slot * kRedBlocks);
+        finish(c, slot, 1);
     }
     void polyakov(const Ctx& c, const void* U, int slot) const override
     {
@@ -264,7 +288,7 @@ public:
     }
     void wilson_square(const Ctx& c, const void* C, int L, int slot) const override
     {
-        k_wilson_square<<<kRedBlocks, kRedThreads, 0, c.stream>>>(full64(C, c.g), c.g, L,
+        k_wilson_square<<<kRedBlocks, 192, 0, c.stream>>>(full64(C, c.g), c.g, L,
                                                                    c.partials + (size_t)slot * kRedBlocks);
         finish(c, slot, 1);
     }

@@ -2006,8 +2006,9 @@ __global__ void __launch_bounds__(4 * kSitesPerBlock, LT_MINB_STAGED)
 }
 
 // The second half of a split flow stage: Z <- c_old Z + c_new X, U' = exp(c_exp Z) U, with
-// X = Algebra(st U^dag) from k_flow_force.  FP64 links run the stage as these two kernels:
-// the fused stage needs 254 registers (two blocks of 128 per SM), the halves far fewer each.
+// X = Algebra(st U^dag) from k_flow_force.  FP64 links run a rectangle stage (and, where there is no
+// memory for the plaquette planes, a Wilson stage) as these two kernels: the fused stage needs 254
+// registers (two blocks of 128 per SM), the halves far fewer each.
 template <typename T, int NR>
 __global__ void __launch_bounds__(kThreads) k_flow_update(Gauge<T, NR> Uin, Gauge<T, NR> Uout, Alg<T> Z, Alg<T> X,
                                                           Geom g, T c_old, T c_new, T c_exp, int read_z, int write_z,
@@ -2162,6 +2163,105 @@ LT_D auto clover_leaves(const F& U, const Geom& g, int par, int i, const int c[4
 // (observables/field_strength_tensor.hpp:28-66, :107-134, :154-175).
 // Products run in FP64 for every storage: the cancellations in F = C - C^dag of a smooth
 // (flowed) field would otherwise lift FP32 rounding of the leaves into Q and E.
+//
+// A block is six planes (warps) of 32 sites: each thread multiplies out the four leaves of one plane, takes
+// its share of e, and the planes' H = -i F meet in shared memory, where three warps take the dual pairs of q.
+// One thread a site needed 254 registers for all six planes one after the other and gave an 8^4
+// lattice sixteen blocks.  Bound by the links that come through L2 and, on FP32 storage, by their
+// conversion.  A call for Q and E before and now: FP64 8^4 55 and 33 us, 32 x 24^3 451 and 419; FP32 32^4 963 and
+// 904; two-row FP32 8^4 57 and 33, larger lattices below.  Plaquette, Q and E after a flow step: FP64
+// 8^4 138 and 82 us with the step, two-row FP32 32^4 2319 and 2144.
+//
+// Block (bx, t): timeslice t, or with one row of blocks the whole lattice.  partials: q, e and, with
+// WITH_PLAQ, the plaquette sum, gridDim.y rows of gridDim.x each.
+// The nine reals (herm9_scale) of -i (C - C^dag) of the plane (mu, nu), the leaves of clover_leaves one
+// after the other (the fences keep the loads of the next from being held through this one); plaq: Re tr of the
+// first, the plaquette
+template <typename F>
+LT_D void clover_herm9(const F& U, const Geom& g, int par, int i, const int c[4], int mu, int nu, double h[9], double& plaq)
+{
+    const int op = par ^ 1, s = i >> 1;
+    const int up_mu = step_up_rt(g, mu, c), up_nu = step_up_rt(g, nu, c), dn_nu = step_dn_rt(g, nu, c);
+    const int im = i + step_dn_rt(g, mu, c), in = i + dn_nu, imn = im + dn_nu;
+#pragma unroll
+    for (int q = 0; q < 9; ++q) h[q] = 0.0;
+    {
+        const auto a = mul(U.ld(mu, par, s), U.ld(nu, op, (i + up_mu) >> 1));
+        const auto b = mul(U.ld(nu, par, s), U.ld(mu, op, (i + up_nu) >> 1));
+        herm9_acc<true>(h, a, b);
+        plaq = retr_nd(a, b);
+    }
+    asm volatile("" ::: "memory");
+    herm9_acc<false>(h, mul_nd(U.ld(nu, par, s), U.ld(mu, par, (im + up_nu) >> 1)),
+                     mul_dn(U.ld(nu, op, im >> 1), U.ld(mu, op, im >> 1)));
+    asm volatile("" ::: "memory");
+    herm9_acc<false>(h, mul_dd(U.ld(mu, op, im >> 1), U.ld(nu, par, imn >> 1)),
+                     mul(U.ld(mu, par, imn >> 1), U.ld(nu, op, in >> 1)));
+    asm volatile("" ::: "memory");
+    herm9_acc<true>(h, mul(mul_dn(U.ld(nu, op, in >> 1), U.ld(mu, op, in >> 1)), U.ld(nu, par, (in + up_mu) >> 1)),
+                    U.ld(mu, par, s));
+    herm9_scale(h);
+}
+
+template <int Unused = 0> LT_D int plane_lo(int pl) { return pl < 3 ? 0 : pl < 5 ? 1 : 2; }
+template <int Unused = 0> LT_D int plane_hi(int pl) { return pl < 3 ? pl + 1 : pl < 5 ? pl - 1 : 3; }
+
+template <typename T, int NR, bool WITH_PLAQ>
+__global__ void __launch_bounds__(192, 2) k_clover_obs(Gauge<T, NR> Ust, Geom g, double* __restrict__ partials)
+{
+    __shared__ double sh[32];
+    __shared__ double hs[6][9][32];
+    const Widened<T, NR> U{ Ust };
+    const int lane = threadIdx.x & 31, pl = threadIdx.x >> 5;
+    // sites of the block's row: those of one parity, then the other (a timeslice holds as many of each)
+    const int n = g.V / gridDim.y, h = n >> 1, first = blockIdx.y * h;
+    Kahan kq, ke, kp;
+    for (int k0 = blockIdx.x * kSitesPerBlock; k0 < n; k0 += gridDim.x * kSitesPerBlock)
+    {
+        const int k = k0 + lane;
+        if (k < n)
+        {
+            const int par = k >= h;
+            int c[4];
+            const int i = site_coords(g, par, first + k - par * h, c);
+            double v[9], p;
+            clover_herm9(U, g, par, i, c, plane_lo<>(pl), plane_hi<>(pl), v, p);
+            if (WITH_PLAQ) kp.add(p);
+            const double tr = v[0] + v[1] + v[2];
+            double e = -tr * tr * (1.0 / 3.0);
+#pragma unroll
+            for (int q = 0; q < 9; ++q)
+            {
+                e += v[q] * v[q];
+                hs[pl][q][lane] = v[q];
+            }
+            ke.add(e * (1.0 / 64.0));
+        }
+        __syncthreads();
+        if (pl < 3 && k < n)
+        {
+            double t = 0.0;   // ReTr(F F') = -tr(H H')
+#pragma unroll
+            for (int q = 0; q < 9; ++q) t -= hs[pl][q][lane] * hs[5 - pl][q][lane];
+            kq.add(pl == 1 ? -t : t);
+        }
+        __syncthreads();
+    }
+    const double rq = block_sum(kq.s - kq.c, sh), re = block_sum(ke.s - ke.c, sh);
+    const double rp = WITH_PLAQ ? block_sum(kp.s - kp.c, sh) : 0.0;
+    if (threadIdx.x == 0)
+    {
+        double* out = partials + (size_t)blockIdx.y * gridDim.x + blockIdx.x;
+        const size_t row = (size_t)gridDim.y * gridDim.x;
+        out[0] = rq;
+        out[row] = re;
+        if (WITH_PLAQ) out[2 * row] = rp;
+    }
+}
+
+// One thread a site, for two-row links from 16^4 on: it loads (and rebuilds and widens) each link of a plane
+// once where the fenced leaves of k_clover_obs load some twice (32^4: 878 us against 913, timeslices 888
+// against 918; 16^4 82 and 90 for timeslices; below that k_clover_obs, 8^4 33 us against 57).
 // Unnormalised clover densities of one site: q = ReTr(F01 F23 - F02 F13 + F03 F12) and
 // e = sum_{mu<nu} ReTr(F~^2) with F = C - C^dag, F~ = Traceless(-i/8 F)
 template <typename T, int NR>
@@ -2200,7 +2300,7 @@ LT_D void clover_densities(const Widened<T, NR>& U, const Geom& g, int par, int 
 }
 
 template <typename T, int NR>
-__global__ void __launch_bounds__(kRedThreads) k_clover_obs(Gauge<T, NR> Ust, Geom g, double* __restrict__ partials)
+__global__ void __launch_bounds__(kRedThreads) k_clover_site(Gauge<T, NR> Ust, Geom g, double* __restrict__ partials)
 {
     __shared__ double sh[32];
     const Widened<T, NR> U{ Ust };
@@ -2345,26 +2445,23 @@ __global__ void __launch_bounds__(kRedThreads) k_clover_timeslice(Gauge<T, NR> U
     }
 }
 
-// Per site over the six planes mu < nu: the plaquette traces (slot 0), the 1x2 and 2x1 loop
+// Per site over the six planes mu < nu: the plaquette traces (slot 0) and the 1x2 and 2x1 loop
 // traces of Rectangular<2>::Action (slot 1; rectangular_action.hpp:61-94, wilson_loop.hpp:155-175)
-// and the plaquette charge density of TopChargePlaquette (slot 2; topological_charge.hpp:366-416)
 template <typename T, int NR>
 __global__ void __launch_bounds__(kRedThreads) k_loops(Gauge<T, NR> Ust, Geom g, double* __restrict__ partials)
 {
     __shared__ double sh[32];
     const Widened<T, NR> U{ Ust };
-    Kahan kp, kr, kq;
+    Kahan kp, kr;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < g.V; i += gridDim.x * blockDim.x)
     {
         int c[4];
         const int par = coords_of(g, i, c), op = par ^ 1;
-        M3<double> F[6];
         double sp = 0.0, sr = 0.0;
-        int pl = 0;
 #pragma unroll 1
         for (int mu = 0; mu < 4; ++mu)
 #pragma unroll 1
-            for (int nu = mu + 1; nu < 4; ++nu, ++pl)
+            for (int nu = mu + 1; nu < 4; ++nu)
             {
                 const int imu = shifted(g, c, mu, 1), inu = shifted(g, c, nu, 1);
                 int cmu[4], cnu[4];
@@ -2377,7 +2474,6 @@ __global__ void __launch_bounds__(kRedThreads) k_loops(Gauge<T, NR> Ust, Geom g,
                 const M3<double> a = mul(umu, unu_mu);
                 const M3<double> p = mul_nd(a, mul(unu, umu_nu));
                 sp += p.e[0][0].r + p.e[1][1].r + p.e[2][2].r;
-                F[pl] = p - adj(p);   // times -i below
                 // 1x2: U_mu(x) U_nu(x+mu) U_nu(x+mu+nu) U_mu(x+2nu)^dag U_nu(x+nu)^dag U_nu(x)^dag
                 const M3<double> r12 = mul_nd(mul(a, U.ld(nu, par, imunu >> 1)),
                                               mul(mul(unu, U.ld(nu, op, inu >> 1)), U.ld(mu, par, inu2 >> 1)));
@@ -2386,22 +2482,55 @@ __global__ void __launch_bounds__(kRedThreads) k_loops(Gauge<T, NR> Ust, Geom g,
                                               mul(mul(unu, umu_nu), U.ld(mu, par, imunu >> 1)));
                 sr += r12.e[0][0].r + r12.e[1][1].r + r12.e[2][2].r + r21.e[0][0].r + r21.e[1][1].r + r21.e[2][2].r;
             }
-        // F_mu,nu = -i (P - P^dag); Re tr(F01 F23 + F02 F31 + F03 F12) with F31 = -F13 and
-        // (-i)^2 = -1: -(G01 G23 - G02 G13 + G03 G12) for G = P - P^dag (planes 01 02 03 12 13 23)
-        const double q = -(retr_mul(F[0], F[5]) - retr_mul(F[1], F[4]) + retr_mul(F[2], F[3]));
         kp.add(sp);
         kr.add(sr);
-        kq.add(q);
     }
     double a = block_sum(kp.s - kp.c, sh);
     double b = block_sum(kr.s - kr.c, sh);
-    double d = block_sum(kq.s - kq.c, sh);
     if (threadIdx.x == 0)
     {
         partials[blockIdx.x] = a;
         partials[gridDim.x + blockIdx.x] = b;
-        partials[2 * gridDim.x + blockIdx.x] = d;
     }
+}
+
+// The plaquette charge density of TopChargePlaquette (topological_charge.hpp:366-416), a block six planes
+// of 32 sites as k_clover_obs.  With F = -i (P - P^dag) = H: Re tr(F01 F23 + F02 F31 + F03 F12), F31 = -F13.
+template <typename T, int NR>
+__global__ void __launch_bounds__(192) k_plaq_charge(Gauge<T, NR> Ust, Geom g, double* __restrict__ partials)
+{
+    __shared__ double sh[32];
+    __shared__ double hs[6][9][32];
+    const Widened<T, NR> U{ Ust };
+    const int lane = threadIdx.x & 31, pl = threadIdx.x >> 5, mu = plane_lo<>(pl), nu = plane_hi<>(pl);
+    Kahan k;
+    for (int x0 = blockIdx.x * kSitesPerBlock; x0 < g.V; x0 += gridDim.x * kSitesPerBlock)
+    {
+        const int x = x0 + lane;
+        if (x < g.V)
+        {
+            const int par = x >= g.vh, s = x - par * g.vh, op = par ^ 1;
+            int c[4];
+            const int i = site_coords(g, par, s, c);
+            double v[9] = { 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0 };
+            herm9_acc<true>(v, mul(U.ld(mu, par, s), U.ld(nu, op, (i + step_up_rt(g, mu, c)) >> 1)),
+                            mul(U.ld(nu, par, s), U.ld(mu, op, (i + step_up_rt(g, nu, c)) >> 1)));
+            herm9_scale(v);
+#pragma unroll
+            for (int e = 0; e < 9; ++e) hs[pl][e][lane] = v[e];
+        }
+        __syncthreads();
+        if (pl < 3 && x < g.V)
+        {
+            double t = 0.0;
+#pragma unroll
+            for (int e = 0; e < 9; ++e) t += hs[pl][e][lane] * hs[5 - pl][e][lane];
+            k.add(pl == 1 ? -t : t);
+        }
+        __syncthreads();
+    }
+    const double r = block_sum(k.s - k.c, sh);
+    if (threadIdx.x == 0) partials[blockIdx.x] = r;
 }
 
 // Straight line products for WilsonLoop (observables/wilson_loop.hpp:63-124), kept as full
@@ -2454,36 +2583,23 @@ __global__ void k_chain_double(Full<double> Cin, Full<double> Cout, Geom g, int 
     Cout.st(mu, par, s, mul(Cin.ld(mu, par, s), Cin.ld(mu, pj, j >> 1)));
 }
 
-// sum over sites and mu < nu of Re tr(C_mu(x) C_nu(x+L mu) C_mu(x+L nu)^dag C_nu(x)^dag)
+// sum over sites and mu < nu of Re tr(C_mu(x) C_nu(x+L mu) C_mu(x+L nu)^dag C_nu(x)^dag); a block is six
+// planes (warps) of 32 sites
 template <int Unused = 0>
-__global__ void __launch_bounds__(kRedThreads) k_wilson_square(Full<double> C, Geom g, int L, double* __restrict__ partials)
+__global__ void __launch_bounds__(192) k_wilson_square(Full<double> C, Geom g, int L, double* __restrict__ partials)
 {
     __shared__ double sh[32];
+    const int pl = threadIdx.x >> 5, mu = plane_lo<>(pl), nu = plane_hi<>(pl);
     Kahan k;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < g.V; i += gridDim.x * blockDim.x)
+    for (int x = blockIdx.x * kSitesPerBlock + (threadIdx.x & 31); x < g.V; x += gridDim.x * kSitesPerBlock)
     {
+        const int par = x >= g.vh, s = x - par * g.vh;
         int c[4];
-        const int par = coords_of(g, i, c);
-        double w = 0.0;
-#pragma unroll 1
-        for (int mu = 0; mu < 4; ++mu)
-        {
-            const M3<double> cmu = C.ld(mu, par, i >> 1);
-            const int jm = shifted(g, c, mu, L);
-            int cm[4];
-            const int pm = coords_of(g, jm, cm);
-#pragma unroll 1
-            for (int nu = mu + 1; nu < 4; ++nu)
-            {
-                const int jn = shifted(g, c, nu, L);
-                int cn[4];
-                const int pn = coords_of(g, jn, cn);
-                const M3<double> a = mul(cmu, C.ld(nu, pm, jm >> 1));
-                const M3<double> b = mul(C.ld(nu, par, i >> 1), C.ld(mu, pn, jn >> 1));
-                w += retr_nd(a, b);
-            }
-        }
-        k.add(w);
+        site_coords(g, par, s, c);
+        const int pj = par ^ (L & 1), sm = shifted(g, c, mu, L) >> 1, sn = shifted(g, c, nu, L) >> 1;
+        const M3<double> a = mul(C.ld(mu, par, s), C.ld(nu, pj, sm));
+        const M3<double> b = mul(C.ld(nu, par, s), C.ld(mu, pj, sn));
+        k.add(retr_nd(a, b));
     }
     double r = block_sum(k.s - k.c, sh);
     if (threadIdx.x == 0) partials[blockIdx.x] = r;

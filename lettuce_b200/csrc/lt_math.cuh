@@ -397,6 +397,44 @@ template <bool UP, typename T> LT_HD M3<T> conjugate_h(const M3<T>& h, const M3<
     return r;
 }
 
+// h += the nine reals of -i (P - P^dag) for P = A B (DB: A B^dag), diagonal, then upper entries,
+// without forming P: h_i = 2 Im P_ii; Im P_ij + Im P_ji, Re P_ji - Re P_ij
+template <bool DB, typename T> LT_HD void herm9_acc(T h[9], const M3<T>& a, const M3<T>& b)
+{
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+    {
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int j = 0; j < 3; ++j)
+            {
+                const T xr = a.e[i][k].r, xi = a.e[i][k].i;
+                const T yr = DB ? b.e[j][k].r : b.e[k][j].r, yi = DB ? -b.e[j][k].i : b.e[k][j].i;
+                const int q = i == j ? i : 3 + 2 * (i + j - 1);
+                h[q] += xr * yi;
+                h[q] += xi * yr;
+                if (i < j)
+                {
+                    h[q + 1] -= xr * yr;
+                    h[q + 1] += xi * yi;
+                }
+                else if (i > j)
+                {
+                    h[q + 1] += xr * yr;
+                    h[q + 1] -= xi * yi;
+                }
+            }
+    }
+}
+// Its final scale: the diagonal doubled and the upper entries times sqrt 2, so that tr(H H') is the dot
+// product of the nine
+template <typename T> LT_HD void herm9_scale(T h[9])
+{
+#pragma unroll
+    for (int q = 0; q < 9; ++q) h[q] *= q < 3 ? (T)2 : (T)1.41421356237309504880;
+}
+
 // ---------------------------------------------------------------- reunitarisation
 // RestoreLastRow (math/su3.hpp:362-367): row 2 = conj(row 0 x row 1)
 // g1 a + g2 b as an FMA chain
