@@ -214,7 +214,18 @@ constexpr FlowStage kRK3W7[] = { { 0.0, 1.0, 1.0 / 3.0, 0, 1 },
                                  { -25.0 / 48.0, 15.0 / 16.0, 1.0, 1, 1 },
                                  { -17.0 / 25.0, 8.0 / 15.0, 1.0, 1, 0 } };
 
-int flow_steps(lt_lattice* h, double eps, int n_step, int integrator = LT_FLOW_RK3)
+// The context of a force on links as they are given (uploaded, loaded, copied): the planes' lower staples and
+// the conjugated Lambdas take links for unitary, which those of a file of FP32 accuracy are not to
+// FP64.  Flow stages, drifts and stout levels project what they write to the storage's rounding.
+lt::Ctx ctx_given(const lt_lattice* h)
+{
+    lt::Ctx c = h->ctx();
+    c.planes = nullptr;
+    return c;
+}
+
+// given: h->U has not been through a stage of this flow yet
+int flow_steps(lt_lattice* h, double eps, int n_step, int integrator = LT_FLOW_RK3, bool given = true)
 {
     const FlowStage* st = integrator == LT_FLOW_EULER ? kEuler
                         : integrator == LT_FLOW_RK2   ? kRK2
@@ -223,13 +234,14 @@ int flow_steps(lt_lattice* h, double eps, int n_step, int integrator = LT_FLOW_R
     LT_TRY(ensure(h, &h->U2, h->be->gauge_bytes(h->g)));
     if (ns > 1) LT_TRY(ensure(h, &h->Z, h->be->alg_bytes(h->g)));
     const bool zeuthen = h->flow_action == LT_FLOW_ACTION_ZEUTHEN;
-    ensure_force(h, zeuthen || h->act_radius == 2);
-    const bool split = h->be->flow_split() && (h->act_radius == 2 || !h->planes);
+    const bool split = h->be->flow_split();
     if (zeuthen || split) LT_TRY(ensure(h, &h->Xz, h->be->alg_bytes(h->g)));
-    const lt::Ctx c = h->ctx();
+    ensure_force(h, zeuthen || h->act_radius == 2);
     for (int k = 0; k < n_step; ++k)
         for (int j = 0; j < ns; ++j)
         {
+            const lt::Ctx c = given ? ctx_given(h) : h->ctx();
+            given = false;
             if (zeuthen)
                 // the Zeuthen flow's force is that of the Luescher-Weisz action whatever the
                 // handle's gauge action (c_plaq = 5/3, c_rect = -1/12)
@@ -323,7 +335,7 @@ int charge_from_R(lt_lattice* h, double* q)
     return LT_OK;
 }
 
-int metad_backward(lt_lattice* h, double rho, int n_stout, double dvdq, bool have_R = false)
+int metad_backward(lt_lattice* h, double rho, int n_stout, double dvdq, bool given, bool have_R = false)
 {
     LT_TRY(ensure(h, &h->F, h->be->alg_bytes(h->g)));
     LT_TRY(ensure(h, &h->Lam, h->be->alg_bytes(h->g)));
@@ -333,8 +345,9 @@ int metad_backward(lt_lattice* h, double rho, int n_stout, double dvdq, bool hav
     const void* top = level(h, n_stout);
     // scratch that halves the derivative's products on smeared links and, for FP32 links, takes a fifth of the
     // recursion's (in FP64 the Lambda kernel, at its register limit, loses as much); where there is no memory
-    // both do without.  The links as given (no smearing) keep the direct products: the corner sums take
-    // links for unitary, as every smeared level is.
+    // both do without.  Links as given (ctx_given) keep the direct products, in the derivative without smearing
+    // and in the recursion's last level: the corner sums and the conjugated Lambdas take links for unitary,
+    // as every smeared level is.
     if (n_stout > 0)
     {
         (void)try_ensure(h, &h->corners, h->be->corner_bytes(h->g));
@@ -343,8 +356,9 @@ int metad_backward(lt_lattice* h, double rho, int n_stout, double dvdq, bool hav
     h->be->clover_deriv(c, top, h->R, n_stout > 0 ? h->corners : nullptr, h->F, dvdq);
     for (int k = n_stout; k > 0; --k)
     {
-        h->be->stout_lambda(c, level(h, k - 1), level(h, k), h->F, h->Lam, h->Lt, h->Tloc, rho, h->staples[k - 1]);
-        h->be->stout_recursion(c, level(h, k - 1), h->Lam, h->Lt, h->Tloc, h->F, rho);
+        void* Lt = k == 1 && given ? nullptr : h->Lt;
+        h->be->stout_lambda(c, level(h, k - 1), level(h, k), h->F, h->Lam, Lt, h->Tloc, rho, h->staples[k - 1]);
+        h->be->stout_recursion(c, level(h, k - 1), h->Lam, Lt, h->Tloc, h->F, rho);
     }
     return launched("metad_backward");
 }
@@ -385,33 +399,35 @@ struct MetaDParams
 // dV/dQ * dQ/dU into h->F at the current links (CalculateTopologicalForce,
 // updates/hmc_metadynamics.hpp:374-436); with submeasure the CV is recorded as the
 // reference's path samples are (:405-412)
-int metad_force_now(lt_lattice* h, const MetaDParams* md, bool submeasure)
+int metad_force_now(lt_lattice* h, const MetaDParams* md, bool submeasure, bool given)
 {
     LT_TRY(metad_forward(h, md->rho, md->n_stout));
     LT_TRY(metad_clover(h, md->n_stout));
     double q;
     LT_TRY(charge_from_R(h, &q));
     if (submeasure && md->samples) md->samples->push_back(q);
-    return metad_backward(h, md->rho, md->n_stout, md->bias->derivative(q), true);
+    return metad_backward(h, md->rho, md->n_stout, md->bias->derivative(q), given, true);
 }
 
-// With drift_eps set, the drift of that length follows in the same kernel.
-int kick(lt_lattice* h, double beta, double eps, const MetaDParams* md, bool submeasure,
+// given: no drift has projected the links yet (ctx_given).  With drift_eps set, the drift of that length
+// follows in the same kernel.
+int kick(lt_lattice* h, double beta, double eps, const MetaDParams* md, bool submeasure, bool given,
          const double* drift_eps = nullptr)
 {
     const void* F = nullptr;
     if (md)
     {
-        LT_TRY(metad_force_now(h, md, submeasure));
+        LT_TRY(metad_force_now(h, md, submeasure, given));
         F = h->F;
     }
+    const lt::Ctx c = given ? ctx_given(h) : h->ctx();
     if (drift_eps)
     {
-        h->be->md_step(h->ctx(), h->U, h->U2, h->P, F, beta / 6.0, eps, *drift_eps);
+        h->be->md_step(c, h->U, h->U2, h->P, F, beta / 6.0, eps, *drift_eps);
         std::swap(h->U, h->U2);
         return launched("md_step");
     }
-    h->be->momenta(h->ctx(), h->U, h->P, F, beta / 6.0, eps);
+    h->be->momenta(c, h->U, h->P, F, beta / 6.0, eps);
     return launched("momenta");
 }
 
@@ -580,33 +596,36 @@ int integrate(lt_lattice* h, double beta, const std::vector<MdOp>& ops, const Me
     // a kick and the drift after it run together where the storage and the action have that and
     // there is memory for the second link field
     const bool fused = h->be->md_fused(c) && try_ensure(h, &h->U2, h->be->gauge_bytes(h->g));
+    const bool fused_given = fused && h->be->md_fused(ctx_given(h));
+    bool given = true;
     for (size_t k = 0; k < ops.size(); ++k)
     {
         const MdOp& op = ops[k];
         const double* drift_eps = nullptr;
-        if (fused && (op.kind == Md::KICK || op.kind == Md::KICK_GAUGE) && k + 1 < ops.size() &&
-            ops[k + 1].kind == Md::DRIFT)
+        if ((given ? fused_given : fused) && (op.kind == Md::KICK || op.kind == Md::KICK_GAUGE) &&
+            k + 1 < ops.size() && ops[k + 1].kind == Md::DRIFT)
             drift_eps = &ops[++k].eps;
         switch (op.kind)
         {
-        case Md::KICK: LT_TRY(kick(h, beta, op.eps, md, op.sub, drift_eps)); break;
-        case Md::KICK_GAUGE: LT_TRY(kick(h, beta, op.eps, nullptr, false, drift_eps)); break;
+        case Md::KICK: LT_TRY(kick(h, beta, op.eps, md, op.sub, given, drift_eps)); break;
+        case Md::KICK_GAUGE: LT_TRY(kick(h, beta, op.eps, nullptr, false, given, drift_eps)); break;
         case Md::KICK_METAD:
-            LT_TRY(metad_force_now(h, md, op.sub));
+            LT_TRY(metad_force_now(h, md, op.sub, given));
             h->be->alg_axpby(c, h->P, h->F, 1.0, op.eps);
             LT_TRY(launched("metad momenta"));
             break;
         case Md::FRICTION_PRE:
             h->be->alg_axpby(c, h->P, nullptr, std::exp(-op.friction * op.eps), 0.0);
-            LT_TRY(kick(h, beta, op.eps, nullptr, false));
+            LT_TRY(kick(h, beta, op.eps, nullptr, false, given));
             break;
         case Md::FRICTION_POST:
-            LT_TRY(kick(h, beta, op.eps, nullptr, false));
+            LT_TRY(kick(h, beta, op.eps, nullptr, false, given));
             h->be->alg_axpby(c, h->P, nullptr, std::exp(-op.friction * op.eps), 0.0);
             LT_TRY(launched("friction"));
             break;
         case Md::DRIFT: LT_TRY(drift(h, op.eps)); break;
         }
+        if (drift_eps || op.kind == Md::DRIFT) given = false;
     }
     return LT_OK;
 }
@@ -1651,7 +1670,7 @@ int lt_flow_rk3_measure(lt_lattice* in, lt_lattice* out, double eps, int n_meas,
     LT_TRY(lt_copy(out, in));
     for (int m = 0; m < n_meas; ++m)
     {
-        LT_TRY(flow_steps(out, eps, every));
+        LT_TRY(flow_steps(out, eps, every, LT_FLOW_RK3, m == 0));
         if (q_out || e_out)
             LT_TRY(clover_q_e(out, out->U, q_out ? &q_out[m] : nullptr, e_out ? &e_out[m] : nullptr,
                               plaq_out ? &plaq_out[m] : nullptr));
@@ -1672,7 +1691,7 @@ int lt_flow_t0(lt_lattice* in, lt_lattice* out, double eps, double target, int m
     double t_prev = 0.0, y_prev = 0.0, q = 0.0, e = 0.0;
     for (int k = 1; k <= max_steps; ++k)
     {
-        LT_TRY(flow_steps(out, eps, 1));
+        LT_TRY(flow_steps(out, eps, 1, LT_FLOW_RK3, k == 1));
         LT_TRY(clover_q_e(out, out->U, &q, &e));
         const double t = k * eps, y = t * t * e;
         if (y >= target)
@@ -1707,11 +1726,7 @@ int lt_gauge_force(lt_lattice* h, double beta, double* force_out)
     LT_TRY(ensure(h, &h->F, h->be->alg_bytes(h->g)));
     LT_CK(cudaMemsetAsync(h->F, 0, h->be->alg_bytes(h->g), h->stream));
     if (h->act_radius == 2) ensure_force(h, true);
-    // the force of the links as they are given: the planes' lower staples take them for unitary, which links
-    // read from a file of FP32 accuracy are not to FP64
-    lt::Ctx c = h->ctx();
-    c.planes = nullptr;
-    h->be->momenta(c, h->U, h->F, nullptr, beta / 6.0, 1.0);
+    h->be->momenta(ctx_given(h), h->U, h->F, nullptr, beta / 6.0, 1.0);
     LT_TRY(ensure_aos(h));
     h->be->alg_to_aos(h->ctx(), h->F, h->d_aos);
     LT_TRY(launched("lt_gauge_force"));
@@ -1811,7 +1826,7 @@ int lt_clover_derivative(lt_lattice* h, double* out)
     LT_TRY(check_h(h, "lt_clover_derivative"));
     const lt::DeviceScope device_scope(h->device);
     if (!out) return lt::set_error(LT_ERR_ARG, "lt_clover_derivative: null pointer");
-    LT_TRY(metad_backward(h, 0.0, 0, 1.0));
+    LT_TRY(metad_backward(h, 0.0, 0, 1.0, true));
     LT_TRY(ensure_aos(h));
     h->be->alg_to_aos(h->ctx(), h->F, h->d_aos);
     LT_TRY(launched("lt_clover_derivative"));
@@ -1838,7 +1853,7 @@ int lt_metad_force(lt_lattice* h, double rho, int n_stout, double dvdq, double* 
     // the charge is summed before the backward chain but read after it, so the host does not
     // wait between the two halves of the force
     if (q_out) h->be->topcharge_R(h->ctx(), h->R, 7);
-    LT_TRY(metad_backward(h, rho, n_stout, dvdq, true));
+    LT_TRY(metad_backward(h, rho, n_stout, dvdq, true, true));
     if (q_out)
     {
         double r;
