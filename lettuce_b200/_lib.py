@@ -28,6 +28,7 @@ _pd, _pi, _pu64 = C.POINTER(C.c_double), C.POINTER(C.c_int), C.POINTER(C.c_uint6
 SIGNATURES = {
     "lt_last_error": (C.c_char_p, []),
     "lt_version": (_i, []),
+    "lt_release_memory": (_i, []),
     "lt_create": (_i, [_ip, _i, C.POINTER(_vp)]),
     "lt_destroy": (_i, [_vp]),
     "lt_get_extents": (_i, [_vp, _ip, _pi]),
@@ -60,6 +61,7 @@ SIGNATURES = {
     "lt_su3_exp_test": (_i, [_dp, _dp, _i, _i, _i]),
     "lt_device_arch": (_i, [_pi, _pi]),
     "lt_pack_links_test": (_i, [_ip, _dp, C.POINTER(C.c_float)]),
+    "lt_memory_test": (_i, [_u64, _i, _pu64]),
     "lt_overrelax_sweeps": (_i, [_vp, _i]),
     "lt_heatbath_sweeps": (_i, [_vp, _d, _i, _u64, _pu64]),
     "lt_update_sweeps": (_i, [_vp, _d, _i, _i, _i, _u64, _pu64]),

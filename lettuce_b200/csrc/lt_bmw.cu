@@ -35,7 +35,6 @@ size_t payload_bytes(const lt_lattice* h, int full) { return (size_t)h->g.V * 4 
 int staging(lt_lattice* h)
 {
     if (h->d_aos) return LT_OK;
-    LT_CK(cudaSetDevice(h->device));
     LT_CK(lt::dev_alloc(h->device, (void**)&h->d_aos, (size_t)4 * h->g.V * 18 * sizeof(double)));
     return LT_OK;
 }

@@ -40,22 +40,72 @@ namespace {
 struct DevStore
 {
     std::unordered_map<void*, size_t> size;             // every buffer handed out or kept
-    std::unordered_multimap<size_t, void*> kept;        // buffers of no handle, by size
-    size_t kept_bytes = 0, most = 0;
-    int handles = 0;
+    std::vector<std::pair<size_t, void*>> kept;         // buffers of no handle, by size
+    std::unordered_map<void**, cudaStream_t> idle;      // scratch of live handles, by the pointer that holds it
+    size_t bytes = 0, kept_bytes = 0, most = 0;         // sizes of size and kept; the largest kept_bytes
+    size_t limit = 0;                                   // lt_memory_test
+    bool deny = false;
+    uint64_t freed = 0;                                 // buffers returned so far
+    int handles = 0, borrowed = 0;                      // borrowed: scratch in use by calls
+    std::condition_variable returned;                   // borrowed has become less
 
+    cudaError_t fresh(void** p, size_t n)
+    {
+        if (limit && bytes + n > limit) return cudaErrorMemoryAllocation;
+        const cudaError_t e = cudaMalloc(p, n);
+        if (e != cudaSuccess) return e;
+        size[*p] = n;
+        bytes += n;
+        return e;
+    }
+    void drop(void* p)
+    {
+        const auto k = size.find(p);
+        bytes -= k->second;
+        size.erase(k);
+        cudaFree(p);
+    }
     void give_back()
     {
-        for (auto& k : kept)
-        {
-            size.erase(k.second);
-            cudaFree(k.second);
-        }
+        for (const auto& k : kept) drop(k.second);
         kept.clear();
         kept_bytes = 0;
     }
+    void reclaim()
+    {
+        for (auto s = idle.begin(); s != idle.end();)
+        {
+            cudaStreamCaptureStatus st;   // a stream in capture cannot be waited for
+            if (cudaStreamIsCapturing(s->second, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone)
+            {
+                (void)cudaGetLastError();
+                ++s;
+                continue;
+            }
+            cudaStreamSynchronize(s->second);
+            drop(*s->first);
+            *s->first = nullptr;
+            s = idle.erase(s);
+        }
+    }
+    cudaError_t take(void** p, size_t n)                // a kept buffer of that size, or a fresh one
+    {
+        for (size_t k = kept.size(); k-- > 0;)
+            if (kept[k].first == n)
+            {
+                *p = kept[k].second;
+                kept.erase(kept.begin() + (long)k);
+                kept_bytes -= n;
+                return cudaSuccess;
+            }
+        const cudaError_t e = fresh(p, n);
+        if (e == cudaSuccess || kept.empty()) return e;
+        give_back();
+        return fresh(p, n);
+    }
 };
 std::mutex g_store_mutex;
+thread_local int t_borrowed = 0;   // scratch in use by this thread's calls
 // by device; never destroyed, so that handles freed at process exit still find it
 std::unordered_map<int, DevStore>& stores()
 {
@@ -66,49 +116,111 @@ std::unordered_map<int, DevStore>& stores()
 
 cudaError_t dev_alloc(int device, void** p, size_t bytes)
 {
-    std::lock_guard<std::mutex> lk(g_store_mutex);
+    const DeviceScope device_scope(device);
+    std::unique_lock<std::mutex> lk(g_store_mutex);
     DevStore& st = stores()[device];
-    const auto k = st.kept.find(bytes);
-    if (k != st.kept.end())
+    cudaError_t e = st.take(p, bytes);
+    if (e != cudaSuccess)
     {
-        *p = k->second;
-        st.kept.erase(k);
-        st.kept_bytes -= bytes;
-        return cudaSuccess;
+        st.reclaim();
+        e = st.take(p, bytes);
     }
-    cudaError_t e = cudaMalloc(p, bytes);
-    if (e != cudaSuccess && st.kept_bytes)
+    // scratch that other threads' calls hold comes back with the end of those calls
+    while (e != cudaSuccess && !t_borrowed && st.borrowed)
+    {
+        st.returned.wait(lk);
+        st.reclaim();
+        e = st.take(p, bytes);
+    }
+    if (e != cudaSuccess)
     {
         (void)cudaGetLastError();
-        st.give_back();
-        e = cudaMalloc(p, bytes);
+        *p = nullptr;
     }
-    if (e == cudaSuccess) st.size[*p] = bytes;
-    else *p = nullptr;
     return e;
 }
 
-void dev_free(int device, void* p)
+bool dev_borrow(int device, void** p, size_t bytes, uint64_t* refused)
+{
+    const DeviceScope device_scope(device);
+    std::lock_guard<std::mutex> lk(g_store_mutex);
+    DevStore& st = stores()[device];
+    st.idle.erase(p);
+    if (!*p)
+    {
+        if (st.deny || *refused == st.freed) return false;
+        if (st.take(p, bytes) != cudaSuccess)
+        {
+            (void)cudaGetLastError();
+            *p = nullptr;
+            *refused = st.freed;
+            return false;
+        }
+    }
+    ++st.borrowed;
+    ++t_borrowed;
+    return true;
+}
+
+void dev_lend(int device, void** p, cudaStream_t stream, bool keep)
 {
     std::lock_guard<std::mutex> lk(g_store_mutex);
     DevStore& st = stores()[device];
-    const auto k = st.size.find(p);
-    if (k == st.size.end()) return;
+    if (!keep) st.idle[p] = stream;
+    --st.borrowed;
+    --t_borrowed;
+    st.returned.notify_all();
+}
+
+bool dev_claim(int device, void** p)
+{
+    std::lock_guard<std::mutex> lk(g_store_mutex);
+    stores()[device].idle.erase(p);
+    return *p != nullptr;
+}
+
+void dev_free(int device, void** p)
+{
+    const DeviceScope device_scope(device);
+    std::lock_guard<std::mutex> lk(g_store_mutex);
+    DevStore& st = stores()[device];
+    st.idle.erase(p);
+    if (!*p) return;
     if (!st.most)
     {
         size_t avail = 0, total = 0;
         if (cudaMemGetInfo(&avail, &total) == cudaSuccess) st.most = total / 8;
         else (void)cudaGetLastError();
     }
-    const size_t bytes = k->second;
+    const size_t bytes = st.size[*p];
+    ++st.freed;
     if (st.kept_bytes + bytes > st.most)
+        st.drop(*p);
+    else
     {
-        st.size.erase(k);
-        cudaFree(p);
-        return;
+        st.kept.emplace_back(bytes, *p);
+        st.kept_bytes += bytes;
     }
-    st.kept.emplace(bytes, p);
-    st.kept_bytes += bytes;
+    *p = nullptr;
+}
+
+void dev_release(int device)
+{
+    const DeviceScope device_scope(device);
+    std::lock_guard<std::mutex> lk(g_store_mutex);
+    DevStore& st = stores()[device];
+    st.give_back();
+    st.reclaim();
+}
+
+size_t dev_test(int device, size_t limit, bool deny)
+{
+    std::lock_guard<std::mutex> lk(g_store_mutex);
+    DevStore& st = stores()[device];
+    st.limit = limit;
+    st.most = limit / 8;   // 0: an eighth of the device's memory
+    st.deny = deny;
+    return st.bytes;
 }
 
 void dev_handle_created(int device)
@@ -136,34 +248,71 @@ int check_h(const lt_lattice* h, const char* fn)
 
 int ensure(lt_lattice* h, void** p, size_t bytes)
 {
-    if (*p) return LT_OK;
+    if (lt::dev_claim(h->device, p)) return LT_OK;
     LT_CK(lt::dev_alloc(h->device, p, bytes));
     return LT_OK;
 }
 
-// Scratch that a call can do without: false, with no error left behind, if there is no memory
-bool try_ensure(lt_lattice* h, void** p, size_t bytes)
+// The scratch that a call can do without, borrowed for its duration; after it any allocation that
+// fails may take the memory.  A call allocates what it cannot do without first.
+class Scratch
 {
-    if (*p || lt::dev_alloc(h->device, p, bytes) == cudaSuccess) return true;
-    (void)cudaGetLastError();
-    return false;
-}
-
-// The scratch fields of a force over all links (rect: with rectangles).  On the largest lattices there may
-// be no memory for them; the staples are then multiplied out link by link, as they are without them.
-void ensure_force(lt_lattice* h, bool rect)
-{
-    if (!rect)
+public:
+    explicit Scratch(lt_lattice* h) : h_(h) {}
+    ~Scratch()
     {
-        const size_t bytes = h->be->plane_bytes(h->g);
-        if (bytes) (void)try_ensure(h, &h->planes, bytes);
-        return;
+        // a call that the caller captures into a graph keeps its scratch: the graph holds the addresses
+        cudaStreamCaptureStatus st;
+        if (cudaStreamIsCapturing(h_->stream, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone)
+            h_->captured = true;
+        for (int k = 0; k < n_; ++k) lt::dev_lend(h_->device, slot_[k], h_->stream, h_->captured);
     }
-    if (h->rectE) return;
-    if (try_ensure(h, &h->rectD, h->be->gauge_bytes(h->g)) && try_ensure(h, &h->rectE, h->be->full_bytes(h->g))) return;
-    if (h->rectD) lt::dev_free(h->device, h->rectD);
-    h->rectD = nullptr;
-}
+    Scratch(const Scratch&) = delete;
+    Scratch& operator=(const Scratch&) = delete;
+
+    // false, with no error left behind, if there is no memory
+    bool take(void** p, size_t bytes)
+    {
+        if (!lt::dev_borrow(h_->device, p, bytes, &h_->refused)) return false;
+        slot_[n_++] = p;
+        return true;
+    }
+
+    // The fields of a force over all links (rect: with rectangles).  On the largest lattices there may be
+    // no memory for them; the staples are then multiplied out link by link.
+    void force(bool rect)
+    {
+        const lt::Backend* be = h_->be;
+        if (!rect)
+        {
+            if (const size_t bytes = be->plane_bytes(h_->g)) planes_ = take(&h_->planes, bytes);
+        }
+        else
+            rect_ = take(&h_->rectD, be->gauge_bytes(h_->g)) && take(&h_->rectE, be->full_bytes(h_->g));
+    }
+
+    // The handle's context with the force fields that were taken.  given: for links as they are given
+    // (uploaded, loaded, copied).  The planes' lower staples and the conjugated Lambdas take links for
+    // unitary, which those of a file of FP32 accuracy are not to FP64.  Flow stages, drifts and stout
+    // levels project what they write to the storage's rounding.
+    lt::Ctx ctx(bool given) const
+    {
+        lt::Ctx c = h_->ctx();
+        if (planes_ && !given) c.planes = h_->planes;
+        if (rect_)
+        {
+            c.rectD = h_->rectD;
+            c.rectE = h_->rectE;
+        }
+        return c;
+    }
+
+private:
+    lt_lattice* h_;
+    void** slot_[6];
+    int n_ = 0;
+    bool planes_ = false, rect_ = false;
+};
 
 int ensure_aos(lt_lattice* h) { return ensure(h, (void**)&h->d_aos, (size_t)4 * h->g.V * 18 * sizeof(double)); }
 
@@ -214,16 +363,6 @@ constexpr FlowStage kRK3W7[] = { { 0.0, 1.0, 1.0 / 3.0, 0, 1 },
                                  { -25.0 / 48.0, 15.0 / 16.0, 1.0, 1, 1 },
                                  { -17.0 / 25.0, 8.0 / 15.0, 1.0, 1, 0 } };
 
-// The context of a force on links as they are given (uploaded, loaded, copied): the planes' lower staples and
-// the conjugated Lambdas take links for unitary, which those of a file of FP32 accuracy are not to
-// FP64.  Flow stages, drifts and stout levels project what they write to the storage's rounding.
-lt::Ctx ctx_given(const lt_lattice* h)
-{
-    lt::Ctx c = h->ctx();
-    c.planes = nullptr;
-    return c;
-}
-
 // given: h->U has not been through a stage of this flow yet
 int flow_steps(lt_lattice* h, double eps, int n_step, int integrator = LT_FLOW_RK3, bool given = true)
 {
@@ -236,11 +375,12 @@ int flow_steps(lt_lattice* h, double eps, int n_step, int integrator = LT_FLOW_R
     const bool zeuthen = h->flow_action == LT_FLOW_ACTION_ZEUTHEN;
     const bool split = h->be->flow_split();
     if (zeuthen || split) LT_TRY(ensure(h, &h->Xz, h->be->alg_bytes(h->g)));
-    ensure_force(h, zeuthen || h->act_radius == 2);
+    Scratch scratch(h);
+    scratch.force(zeuthen || h->act_radius == 2);
     for (int k = 0; k < n_step; ++k)
         for (int j = 0; j < ns; ++j)
         {
-            const lt::Ctx c = given ? ctx_given(h) : h->ctx();
+            const lt::Ctx c = scratch.ctx(given);
             given = false;
             if (zeuthen)
                 // the Zeuthen flow's force is that of the Luescher-Weisz action whatever the
@@ -288,7 +428,7 @@ int plaq_of(lt_lattice* h, const void* U, double* out)
 // smearing/stout_smearing.hpp:92-119): the exponential constants are not stored (the adjoint
 // recomputes them), the staple of every level is (the adjoint's Lambda step reads it back
 // instead of computing it again)
-int metad_forward(lt_lattice* h, double rho, int n_stout)
+int metad_levels(lt_lattice* h, int n_stout)
 {
     while ((int)h->levels.size() < n_stout)
     {
@@ -302,6 +442,12 @@ int metad_forward(lt_lattice* h, double rho, int n_stout)
         LT_CK(lt::dev_alloc(h->device, &p, h->be->full_bytes(h->g)));
         h->staples.push_back(p);
     }
+    return LT_OK;
+}
+
+int metad_forward(lt_lattice* h, double rho, int n_stout)
+{
+    LT_TRY(metad_levels(h, n_stout));
     const lt::Ctx c = h->ctx();
     const void* prev = h->U;
     for (int k = 0; k < n_stout; ++k)
@@ -314,8 +460,6 @@ int metad_forward(lt_lattice* h, double rho, int n_stout)
 
 const void* level(const lt_lattice* h, int k) { return k == 0 ? h->U : h->levels[k - 1]; }
 
-// dvdq * dQ/dU into h->F, given the forward chain (CalculateTopologicalForce,
-// updates/hmc_metadynamics.hpp:374-436)
 // The clover planes R of the most smeared level (CalculateClover, hmc_metadynamics.hpp:397-399)
 int metad_clover(lt_lattice* h, int n_stout)
 {
@@ -335,28 +479,35 @@ int charge_from_R(lt_lattice* h, double* q)
     return LT_OK;
 }
 
-int metad_backward(lt_lattice* h, double rho, int n_stout, double dvdq, bool given, bool have_R = false)
+// What the force needs beside the forward chain
+int metad_buffers(lt_lattice* h)
 {
     LT_TRY(ensure(h, &h->F, h->be->alg_bytes(h->g)));
     LT_TRY(ensure(h, &h->Lam, h->be->alg_bytes(h->g)));
     LT_TRY(ensure(h, &h->Tloc, h->be->full_bytes(h->g)));
+    return ensure(h, &h->R, h->be->clov_bytes(h->g));
+}
+
+// dvdq * dQ/dU into h->F, given the forward chain (CalculateTopologicalForce,
+// updates/hmc_metadynamics.hpp:374-436)
+int metad_backward(lt_lattice* h, double rho, int n_stout, double dvdq, bool given, bool have_R = false)
+{
+    LT_TRY(metad_buffers(h));
     if (!have_R) LT_TRY(metad_clover(h, n_stout));
     const lt::Ctx c = h->ctx();
     const void* top = level(h, n_stout);
     // scratch that halves the derivative's products on smeared links and, for FP32 links, takes a fifth of the
     // recursion's (in FP64 the Lambda kernel, at its register limit, loses as much); where there is no memory
-    // both do without.  Links as given (ctx_given) keep the direct products, in the derivative without smearing
-    // and in the recursion's last level: the corner sums and the conjugated Lambdas take links for unitary,
-    // as every smeared level is.
-    if (n_stout > 0)
-    {
-        (void)try_ensure(h, &h->corners, h->be->corner_bytes(h->g));
-        if (h->be->real_bytes() == 4) (void)try_ensure(h, &h->Lt, h->be->alg_bytes(h->g));
-    }
-    h->be->clover_deriv(c, top, h->R, n_stout > 0 ? h->corners : nullptr, h->F, dvdq);
+    // both do without.  Links as given (Scratch::ctx) keep the direct products, in the derivative without
+    // smearing and in the recursion's last level: the corner sums and the conjugated Lambdas take links for
+    // unitary, as every smeared level is.
+    Scratch scratch(h);
+    const bool corners = n_stout > 0 && scratch.take(&h->corners, h->be->corner_bytes(h->g));
+    const bool conj = n_stout > (given ? 1 : 0) && h->be->real_bytes() == 4 && scratch.take(&h->Lt, h->be->alg_bytes(h->g));
+    h->be->clover_deriv(c, top, h->R, corners ? h->corners : nullptr, h->F, dvdq);
     for (int k = n_stout; k > 0; --k)
     {
-        void* Lt = k == 1 && given ? nullptr : h->Lt;
+        void* Lt = conj && !(k == 1 && given) ? h->Lt : nullptr;
         h->be->stout_lambda(c, level(h, k - 1), level(h, k), h->F, h->Lam, Lt, h->Tloc, rho, h->staples[k - 1]);
         h->be->stout_recursion(c, level(h, k - 1), h->Lam, Lt, h->Tloc, h->F, rho);
     }
@@ -409,10 +560,10 @@ int metad_force_now(lt_lattice* h, const MetaDParams* md, bool submeasure, bool 
     return metad_backward(h, md->rho, md->n_stout, md->bias->derivative(q), given, true);
 }
 
-// given: no drift has projected the links yet (ctx_given).  With drift_eps set, the drift of that length
-// follows in the same kernel.
-int kick(lt_lattice* h, double beta, double eps, const MetaDParams* md, bool submeasure, bool given,
-         const double* drift_eps = nullptr)
+// given: no drift has projected the links yet (Scratch::ctx).  With drift_eps set, the drift of that
+// length follows in the same kernel.
+int kick(lt_lattice* h, const Scratch& scratch, double beta, double eps, const MetaDParams* md, bool submeasure,
+         bool given, const double* drift_eps = nullptr)
 {
     const void* F = nullptr;
     if (md)
@@ -420,7 +571,7 @@ int kick(lt_lattice* h, double beta, double eps, const MetaDParams* md, bool sub
         LT_TRY(metad_force_now(h, md, submeasure, given));
         F = h->F;
     }
-    const lt::Ctx c = given ? ctx_given(h) : h->ctx();
+    const lt::Ctx c = scratch.ctx(given);
     if (drift_eps)
     {
         h->be->md_step(c, h->U, h->U2, h->P, F, beta / 6.0, eps, *drift_eps);
@@ -591,12 +742,19 @@ int md_check(int integ, bool metad, const char* fn)
 // Run a program on (h->U, h->P); md null for the gauge action alone
 int integrate(lt_lattice* h, double beta, const std::vector<MdOp>& ops, const MetaDParams* md)
 {
-    ensure_force(h, h->act_radius == 2);
+    // what the forces cannot do without comes before the scratch of this call
+    if (md)
+    {
+        LT_TRY(metad_levels(h, md->n_stout));
+        LT_TRY(metad_buffers(h));
+    }
+    Scratch scratch(h);
+    scratch.force(h->act_radius == 2);
     const lt::Ctx c = h->ctx();
     // a kick and the drift after it run together where the storage and the action have that and
     // there is memory for the second link field
-    const bool fused = h->be->md_fused(c) && try_ensure(h, &h->U2, h->be->gauge_bytes(h->g));
-    const bool fused_given = fused && h->be->md_fused(ctx_given(h));
+    const bool fused = h->be->md_fused(scratch.ctx(false)) && scratch.take(&h->U2, h->be->gauge_bytes(h->g));
+    const bool fused_given = fused && h->be->md_fused(scratch.ctx(true));
     bool given = true;
     for (size_t k = 0; k < ops.size(); ++k)
     {
@@ -607,8 +765,8 @@ int integrate(lt_lattice* h, double beta, const std::vector<MdOp>& ops, const Me
             drift_eps = &ops[++k].eps;
         switch (op.kind)
         {
-        case Md::KICK: LT_TRY(kick(h, beta, op.eps, md, op.sub, given, drift_eps)); break;
-        case Md::KICK_GAUGE: LT_TRY(kick(h, beta, op.eps, nullptr, false, given, drift_eps)); break;
+        case Md::KICK: LT_TRY(kick(h, scratch, beta, op.eps, md, op.sub, given, drift_eps)); break;
+        case Md::KICK_GAUGE: LT_TRY(kick(h, scratch, beta, op.eps, nullptr, false, given, drift_eps)); break;
         case Md::KICK_METAD:
             LT_TRY(metad_force_now(h, md, op.sub, given));
             h->be->alg_axpby(c, h->P, h->F, 1.0, op.eps);
@@ -616,10 +774,10 @@ int integrate(lt_lattice* h, double beta, const std::vector<MdOp>& ops, const Me
             break;
         case Md::FRICTION_PRE:
             h->be->alg_axpby(c, h->P, nullptr, std::exp(-op.friction * op.eps), 0.0);
-            LT_TRY(kick(h, beta, op.eps, nullptr, false, given));
+            LT_TRY(kick(h, scratch, beta, op.eps, nullptr, false, given));
             break;
         case Md::FRICTION_POST:
-            LT_TRY(kick(h, beta, op.eps, nullptr, false, given));
+            LT_TRY(kick(h, scratch, beta, op.eps, nullptr, false, given));
             h->be->alg_axpby(c, h->P, nullptr, std::exp(-op.friction * op.eps), 0.0);
             LT_TRY(launched("friction"));
             break;
@@ -944,6 +1102,23 @@ const char* lt_last_error(void) { return lt::g_last_error.c_str(); }
 
 int lt_version(void) { return 100; }
 
+int lt_release_memory(void)
+{
+    int device = 0;
+    LT_CK(cudaGetDevice(&device));
+    lt::dev_release(device);
+    return LT_OK;
+}
+
+int lt_memory_test(uint64_t limit, int deny_scratch, uint64_t* held)
+{
+    int device = 0;
+    LT_CK(cudaGetDevice(&device));
+    const uint64_t n = lt::dev_test(device, (size_t)limit, deny_scratch != 0);
+    if (held) *held = n;
+    return LT_OK;
+}
+
 int lt_create(const int ext[4], int prec, lt_lattice** out)
 {
     if (!out || !ext) return lt::set_error(LT_ERR_ARG, "lt_create: null pointer");
@@ -1002,13 +1177,12 @@ int lt_destroy(lt_lattice* h)
     // the buffers may serve another handle at once: every use of them on another stream is ordered before
     // this one (ensembles join back, copies and swaps wait)
     if (h->stream) cudaStreamSynchronize(h->stream);
-    void* bufs[] = { h->U,   h->U2,   h->Z,        h->P,       h->F,     h->Ubak,   h->R,      h->chainA,
-                     h->Lam, h->Tloc, h->partials, h->results, h->d_aos, h->status, h->chainB, h->Xz,
-                     h->tensor, h->rectD, h->rectE, h->planes, h->Lt, h->corners };
-    for (void* p : bufs)
-        if (p) lt::dev_free(h->device, p);
-    for (void* p : h->levels) lt::dev_free(h->device, p);
-    for (void* p : h->staples) lt::dev_free(h->device, p);
+    for (void** p : { &h->U, &h->U2, &h->Z, &h->P, &h->F, &h->Ubak, &h->R, &h->Lam, &h->Lt, &h->corners, &h->Tloc,
+                      &h->chainA, &h->chainB, &h->planes, &h->rectD, &h->rectE, &h->Xz, (void**)&h->partials,
+                      (void**)&h->results, (void**)&h->d_aos, (void**)&h->status, (void**)&h->tensor })
+        lt::dev_free(h->device, p);
+    for (void*& p : h->levels) lt::dev_free(h->device, &p);
+    for (void*& p : h->staples) lt::dev_free(h->device, &p);
     if (h->h_results) cudaFreeHost(h->h_results);
     if (h->h_stage) cudaFreeHost(h->h_stage);
     if (h->stream) cudaStreamDestroy(h->stream);
@@ -1724,10 +1898,11 @@ int lt_gauge_force(lt_lattice* h, double beta, double* force_out)
     const lt::DeviceScope device_scope(h->device);
     if (!force_out) return lt::set_error(LT_ERR_ARG, "lt_gauge_force: null pointer");
     LT_TRY(ensure(h, &h->F, h->be->alg_bytes(h->g)));
-    LT_CK(cudaMemsetAsync(h->F, 0, h->be->alg_bytes(h->g), h->stream));
-    if (h->act_radius == 2) ensure_force(h, true);
-    h->be->momenta(ctx_given(h), h->U, h->F, nullptr, beta / 6.0, 1.0);
     LT_TRY(ensure_aos(h));
+    LT_CK(cudaMemsetAsync(h->F, 0, h->be->alg_bytes(h->g), h->stream));
+    Scratch scratch(h);
+    if (h->act_radius == 2) scratch.force(true);
+    h->be->momenta(scratch.ctx(true), h->U, h->F, nullptr, beta / 6.0, 1.0);
     h->be->alg_to_aos(h->ctx(), h->F, h->d_aos);
     LT_TRY(launched("lt_gauge_force"));
     LT_CK(cudaMemcpyAsync(force_out, h->d_aos, (size_t)4 * h->g.V * 18 * sizeof(double), cudaMemcpyDeviceToHost,

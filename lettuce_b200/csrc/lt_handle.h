@@ -11,18 +11,6 @@ namespace lt {
 // Records a CUDA error as this thread's last error; returns LT_ERR_NOMEM or LT_ERR_CUDA.
 int cuda_error(cudaError_t e, const char* what);
 
-// Device memory of the lattice handles.  A handle's buffers go back to a per-device store when it is
-// destroyed and serve the next handle that asks for the same size (a flowed copy made for each
-// measurement, one field after another): a cudaMalloc or cudaFree of a field takes from one to tens of
-// milliseconds, more than most calls that need it (the measurement bundle on one flow level at 32 x 24^3
-// in FP64: 10.3 ms a call with them, 5.1 without).  The store holds at most an eighth of the device's
-// memory, gives everything back when the device's last handle goes, and is emptied and tried again
-// when an allocation fails.  Safe from any thread; dev_free expects no work in flight on the buffer.
-cudaError_t dev_alloc(int device, void** p, size_t bytes);
-void dev_free(int device, void* p);
-void dev_handle_created(int device);
-void dev_handle_gone(int device);
-
 // Makes a handle's device current for one C-ABI call and restores the caller's device after
 struct DeviceScope
 {
@@ -39,6 +27,27 @@ struct DeviceScope
     DeviceScope(const DeviceScope&) = delete;
     DeviceScope& operator=(const DeviceScope&) = delete;
 };
+
+// Device memory of the lattice handles.  A handle's buffers go back to a per-device store when
+// it is destroyed and serve the next handle that asks for the same size (a flowed copy made for each
+// measurement, one field after another): a cudaMalloc or cudaFree of a field takes from one to tens of
+// milliseconds, more than most calls that need it (the measurement bundle on one flow level at 32 x 24^3
+// in FP64: 10.3 ms a call with them, 5.1 without).  The store keeps at most an eighth of the device's memory,
+// and gives everything back when the device's last handle goes.  Scratch that a call
+// can do without is borrowed for the call: after it the buffer stays with its handle, and the pointer that
+// holds it is set to null when the memory is taken.  An allocation that fails empties the store, takes the
+// idle scratch of all handles and waits for the scratch of other threads' calls; borrowing only empties the
+// store, and what was refused is not asked for again until another buffer has been returned.  Safe
+// from any thread.
+cudaError_t dev_alloc(int device, void** p, size_t bytes);
+void dev_free(int device, void** p);    // expects no work in flight on the buffer
+bool dev_borrow(int device, void** p, size_t bytes, uint64_t* refused);
+void dev_lend(int device, void** p, cudaStream_t stream, bool keep);   // ends it; idle once the stream is, or kept
+bool dev_claim(int device, void** p);   // makes an idle buffer the handle's own; false if there is none (any more)
+void dev_release(int device);           // gives back all that no call needs: the store and the lent scratch
+size_t dev_test(int device, size_t limit, bool deny);   // lt_memory_test; returns the bytes held
+void dev_handle_created(int device);
+void dev_handle_gone(int device);
 } // namespace lt
 
 #define LT_CK(call)                                                  \
@@ -100,6 +109,8 @@ struct lt_lattice
     void* rectE = nullptr;       // and their outer staples (full matrices)
     void* Xz = nullptr;          // Luescher-Weisz force of a Zeuthen flow stage (algebra)
     double* tensor = nullptr;    // FullTensor4D of lt_clover_tensor (FP64, reference layout)
+    uint64_t refused = ~0ull;    // state of the store when it had no memory for scratch
+    bool captured = false;       // a call has been captured into a graph: scratch stays
     mutable unsigned order = 0;  // launches of the order-alternating sweep and flow kernels
 
     lt::Ctx ctx() const
@@ -113,9 +124,6 @@ struct lt_lattice
         c.rect = act_radius == 2;
         c.cp = act_cp;
         c.cr = act_cr;
-        c.planes = planes;
-        c.rectD = rectD;
-        c.rectE = rectE;
         c.order = &order;
         return c;
     }
