@@ -40,7 +40,7 @@ namespace {
 struct DevStore
 {
     std::unordered_map<void*, size_t> size;             // every buffer handed out or kept
-    std::vector<std::pair<size_t, void*>> kept;         // buffers of no handle, by size
+    std::vector<std::pair<size_t, void*>> kept;         // buffers of no handle, oldest first
     std::unordered_map<void**, cudaStream_t> idle;      // scratch of live handles, by the pointer that holds it
     size_t bytes = 0, kept_bytes = 0, most = 0;         // sizes of size and kept; the largest kept_bytes
     size_t limit = 0;                                   // lt_memory_test
@@ -65,11 +65,15 @@ struct DevStore
         size.erase(k);
         cudaFree(p);
     }
-    void give_back()
+    void give_back(size_t room = 0)                     // all, or oldest first until room bytes may be kept
     {
-        for (const auto& k : kept) drop(k.second);
-        kept.clear();
-        kept_bytes = 0;
+        size_t n = 0;
+        for (; n < kept.size() && (!room || kept_bytes + room > most); ++n)
+        {
+            kept_bytes -= kept[n].first;
+            drop(kept[n].second);
+        }
+        kept.erase(kept.begin(), kept.begin() + (long)n);
     }
     void reclaim()
     {
@@ -194,10 +198,11 @@ void dev_free(int device, void** p)
     }
     const size_t bytes = st.size[*p];
     ++st.freed;
-    if (st.kept_bytes + bytes > st.most)
+    if (bytes > st.most)
         st.drop(*p);
     else
     {
+        if (st.kept_bytes + bytes > st.most) st.give_back(bytes);
         st.kept.emplace_back(bytes, *p);
         st.kept_bytes += bytes;
     }

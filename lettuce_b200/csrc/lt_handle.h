@@ -33,7 +33,7 @@ struct DeviceScope
 // measurement, one field after another): a cudaMalloc or cudaFree of a field takes from one to tens of
 // milliseconds, more than most calls that need it (the measurement bundle on one flow level at 32 x 24^3
 // in FP64: 10.3 ms a call with them, 5.1 without).  The store keeps at most an eighth of the device's memory,
-// and gives everything back when the device's last handle goes.  Scratch that a call
+// oldest given up first, and gives everything back when the device's last handle goes.  Scratch that a call
 // can do without is borrowed for the call: after it the buffer stays with its handle, and the pointer that
 // holds it is set to null when the memory is taken.  An allocation that fails empties the store, takes the
 // idle scratch of all handles and waits for the scratch of other threads' calls; borrowing only empties the

@@ -214,3 +214,21 @@ def test_threads_at_the_limit():
     for t in threads:
         t.join()
     assert not bad, bad
+
+
+def test_store_keeps_the_newest():
+    """A store that is full gives up its oldest buffers: fields of a size used now stay after fields of a size
+    that is not asked for again have filled it."""
+    small, big = (8, 8, 8, 8), (16, 8, 8, 8)
+    keep = lt.GaugeField((4, 4, 4, 4))
+    nb = 8 * 72 * int(np.prod(small))
+    held(limit=8 * 5 * nb)   # the store keeps an eighth: two big fields' links, or five small ones'
+    old = [lt.GaugeField(big) for _ in range(3)]
+    for f in old:
+        f.close()
+    lt.GaugeField(small).close()
+    before = held(limit=8 * 5 * nb)
+    f = lt.GaugeField(small)   # from the store
+    assert held(limit=8 * 5 * nb) == before
+    f.close()
+    keep.close()
