@@ -53,7 +53,7 @@ int lt_version(void);
 /* Device memory.  Destroyed handles leave their device buffers in a store of at most an eighth of the
  * device's memory, for the next handle of the same size; handles keep scratch fields between calls that
  * they can do without.  Both are taken back when an allocation of this library fails, and the store is
- * emptied with the device's last handle.  lt_release_memory gives both back on the current
+ * emptied with the device's last handle or ensemble.  lt_release_memory gives both back on the current
  * device at once (waiting for the calls that use them), for other allocators of the process. */
 int lt_release_memory(void);
 
@@ -404,7 +404,7 @@ int lt_device_arch(int* binary_version, int* ptx_version);
  * storage: chunk c (0..2) of plane (mu, parity) at ((mu * 2 + parity) * 3 + c) * V/2 float4s,
  * checkerboard index s = site / 2, floats 4c .. 4c + 3 of the link's rows 0-1. */
 int lt_pack_links_test(const int ext[4], const double* links, float* out);
-/* On the current device: allocations of lattices fail that would take the memory they
+/* On the current device: allocations of lattices and ensembles fail that would take the memory they
  * hold above limit bytes (0: no limit); with deny_scratch, scratch fields that calls can do without
  * are refused.  *held (may be NULL): the bytes held now.  Both stay set until the next call. */
 int lt_memory_test(uint64_t limit, int deny_scratch, uint64_t* held);

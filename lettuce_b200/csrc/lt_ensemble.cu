@@ -248,10 +248,12 @@ int lt_ensemble_create(lt_lattice* const* lattices, const double* betas, int n, 
     e->prec = lattices[0]->prec;
     e->device = lattices[0]->device;
     e->be = lattices[0]->be;
+    lt::dev_handle_created(e->device);
     cudaError_t ce = cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking);
-    if (ce == cudaSuccess) ce = cudaMalloc((void**)&e->d_desc, sizeof(lt::LatDesc) * n);
-    if (ce == cudaSuccess) ce = cudaMalloc((void**)&e->d_counter, sizeof(uint64_t));
-    if (ce == cudaSuccess) ce = cudaMalloc((void**)&e->d_bar, (4 + 8 * kMaxRoundSweeps) * sizeof(unsigned));
+    if (ce == cudaSuccess) ce = lt::dev_alloc(e->device, (void**)&e->d_desc, sizeof(lt::LatDesc) * n);
+    if (ce == cudaSuccess) ce = lt::dev_alloc(e->device, (void**)&e->d_counter, sizeof(uint64_t));
+    if (ce == cudaSuccess)
+        ce = lt::dev_alloc(e->device, (void**)&e->d_bar, (4 + 8 * kMaxRoundSweeps) * sizeof(unsigned));
     if (ce == cudaSuccess) ce = cudaMemsetAsync(e->d_bar, 0, 4 * sizeof(unsigned), e->stream);
     if (ce != cudaSuccess)
     {
@@ -275,10 +277,11 @@ int lt_ensemble_destroy(lt_ensemble* e)
     const lt::DeviceScope device_scope(e->device);
     if (e->stream) cudaStreamSynchronize(e->stream);
     drop_graphs(e);
-    if (e->d_desc) cudaFree(e->d_desc);
-    if (e->d_counter) cudaFree(e->d_counter);
-    if (e->d_bar) cudaFree(e->d_bar);
+    lt::dev_free(e->device, (void**)&e->d_desc);
+    lt::dev_free(e->device, (void**)&e->d_counter);
+    lt::dev_free(e->device, (void**)&e->d_bar);
     if (e->stream) cudaStreamDestroy(e->stream);
+    lt::dev_handle_gone(e->device);
     delete e;
     return LT_OK;
 }
@@ -327,14 +330,14 @@ int lt_ensemble_autotune(lt_ensemble* e, int* threads_hb, int* threads_or)
     for (size_t k = 0; k < e->lats.size() && rc == LT_OK; ++k)
     {
         const size_t bytes = e->be->gauge_bytes(e->lats[k]->g);
-        cudaError_t ce = cudaMalloc(&saved[k], bytes);
+        cudaError_t ce = lt::dev_alloc(e->device, &saved[k], bytes);
         if (ce == cudaSuccess) ce = cudaMemcpyAsync(saved[k], e->lats[k]->U, bytes, cudaMemcpyDeviceToDevice, e->stream);
         if (ce != cudaSuccess) rc = lt::cuda_error(ce, "lt_ensemble_autotune: scratch copy");
     }
     uint64_t* d_scratch_counter = nullptr;
     if (rc == LT_OK)
     {
-        cudaError_t ce = cudaMalloc((void**)&d_scratch_counter, sizeof(uint64_t));
+        cudaError_t ce = lt::dev_alloc(e->device, (void**)&d_scratch_counter, sizeof(uint64_t));
         if (ce == cudaSuccess) ce = cudaMemsetAsync(d_scratch_counter, 0, sizeof(uint64_t), e->stream);
         if (ce != cudaSuccess) rc = lt::cuda_error(ce, "lt_ensemble_autotune: counter");
     }
@@ -425,9 +428,8 @@ int lt_ensemble_autotune(lt_ensemble* e, int* threads_hb, int* threads_or)
                             e->stream);
         }
     cudaStreamSynchronize(e->stream);
-    for (void* p : saved)
-        if (p) cudaFree(p);
-    if (d_scratch_counter) cudaFree(d_scratch_counter);
+    for (void*& p : saved) lt::dev_free(e->device, &p);
+    lt::dev_free(e->device, (void**)&d_scratch_counter);
     if (t0) cudaEventDestroy(t0);
     if (t1) cudaEventDestroy(t1);
     if (rc != LT_OK) return rc;

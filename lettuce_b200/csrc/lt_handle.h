@@ -28,12 +28,12 @@ struct DeviceScope
     DeviceScope& operator=(const DeviceScope&) = delete;
 };
 
-// Device memory of the lattice handles.  A handle's buffers go back to a per-device store when
+// Device memory of the lattice handles and ensembles.  A handle's buffers go back to a per-device store when
 // it is destroyed and serve the next handle that asks for the same size (a flowed copy made for each
 // measurement, one field after another): a cudaMalloc or cudaFree of a field takes from one to tens of
 // milliseconds, more than most calls that need it (the measurement bundle on one flow level at 32 x 24^3
 // in FP64: 10.3 ms a call with them, 5.1 without).  The store keeps at most an eighth of the device's memory,
-// oldest given up first, and gives everything back when the device's last handle goes.  Scratch that a call
+// oldest given up first, and gives everything back when the last handle or ensemble goes.  Scratch that a call
 // can do without is borrowed for the call: after it the buffer stays with its handle, and the pointer that
 // holds it is set to null when the memory is taken.  An allocation that fails empties the store, takes the
 // idle scratch of all handles and waits for the scratch of other threads' calls; borrowing only empties the
@@ -46,7 +46,7 @@ void dev_lend(int device, void** p, cudaStream_t stream, bool keep);   // ends i
 bool dev_claim(int device, void** p);   // makes an idle buffer the handle's own; false if there is none (any more)
 void dev_release(int device);           // gives back all that no call needs: the store and the lent scratch
 size_t dev_test(int device, size_t limit, bool deny);   // lt_memory_test; returns the bytes held
-void dev_handle_created(int device);
+void dev_handle_created(int device);    // lattices and ensembles
 void dev_handle_gone(int device);
 } // namespace lt
 

@@ -232,3 +232,22 @@ def test_store_keeps_the_newest():
     assert held(limit=8 * 5 * nb) == before
     f.close()
     keep.close()
+
+
+def test_ensemble_from_the_store():
+    """An ensemble's buffers and the link copies of its tuning come from the store: a destroyed handle's buffers
+    serve them, or give way to them."""
+    keep = [lt.GaugeField((8, 8, 8, 8)) for _ in range(2)]
+    lt.GaugeField((12, 8, 8, 8)).close()
+    before = held()
+    E = lt.Ensemble(keep, [6.0, 6.0], seed=1)
+    assert held() > before
+    lt.GaugeField((8, 8, 8, 8)).close()
+    full = held()
+    held(limit=full)   # the tuning copies 4.7 MB of links: the 2.4 and 3.5 MB of the store
+    E.autotune()
+    assert held() <= full
+    E.sweeps(1)
+    del E
+    for f in keep:
+        f.close()
