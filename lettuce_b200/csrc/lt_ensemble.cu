@@ -217,6 +217,21 @@ int persistent_rounds(lt_ensemble* e, cudaStream_t s, int n_sweep, int n_hb, int
     return LT_OK;
 }
 
+// The rounds of lt_ensemble_sweeps, launched on the ensemble's stream
+int run_rounds(lt_ensemble* e, int n_sweep, int n_hb, int n_or, int reverse, const uint64_t* counter)
+{
+    LT_CK(cudaMemcpyAsync(e->d_counter, counter, sizeof(uint64_t), cudaMemcpyHostToDevice, e->stream));
+    if (e->mode == LT_ENSEMBLE_PERSISTENT)
+        LT_TRY(persistent_rounds(e, e->stream, n_sweep, n_hb, n_or, reverse, e->d_counter));
+    else
+    {
+        cudaGraphExec_t g;
+        LT_TRY(graph_for(e, n_hb, n_or, reverse, &g));
+        for (int k = 0; k < n_sweep; ++k) LT_CK(cudaGraphLaunch(g, e->stream));
+    }
+    return launched("lt_ensemble_sweeps");
+}
+
 } // namespace
 
 extern "C" {
@@ -294,25 +309,14 @@ int lt_ensemble_sweeps(lt_ensemble* e, int n_sweep, int n_hb, int n_or, int reve
     const lt::DeviceScope device_scope(e->device);
     LT_TRY(join_in(e));
     LT_TRY(refresh(e));
-    LT_CK(cudaMemcpyAsync(e->d_counter, counter, sizeof(uint64_t), cudaMemcpyHostToDevice, e->stream));
-    if (e->mode == LT_ENSEMBLE_PERSISTENT)
-    {
-        const int r = persistent_rounds(e, e->stream, n_sweep, n_hb, n_or, reverse ? 1 : 0, e->d_counter);
-        if (r != LT_OK)
-        {
-            join_out(e);
-            return r;
-        }
-    }
-    else
-    {
-        cudaGraphExec_t g;
-        LT_TRY(graph_for(e, n_hb, n_or, reverse ? 1 : 0, &g));
-        for (int k = 0; k < n_sweep; ++k) LT_CK(cudaGraphLaunch(g, e->stream));
-    }
-    LT_TRY(launched("lt_ensemble_sweeps"));
-    LT_TRY(join_out(e));
-    LT_CK(cudaStreamSynchronize(e->stream));
+    const int rc = run_rounds(e, n_sweep, n_hb, n_or, reverse ? 1 : 0, counter);
+    // also after an error: rounds that were launched must be over before a lattice is used or destroyed
+    // (lt_destroy waits for the lattice's own stream and hands its buffers on)
+    const int joined = join_out(e);
+    const cudaError_t waited = cudaStreamSynchronize(e->stream);
+    LT_TRY(rc);
+    LT_TRY(joined);
+    LT_CK(waited);
     *counter += (uint64_t)n_sweep * (uint64_t)n_hb;
     return LT_OK;
 }
