@@ -68,6 +68,7 @@ public:
     // (q then e, nbx blocks per timeslice); plaquette and rectangle sums into
     // results[slot..slot+1]; Polyakov loop re, im into results[slot..slot+1]; straight-line
     // products of the links (full FP64 matrices) for square Wilson loops
+    virtual int clover_block_sites(const Geom& g) const = 0;   // sites that a block of clover_timeslices takes at once
     virtual void clover_timeslices(const Ctx& c, const void* U, double* partials, int nbx) const = 0;
     virtual void loops(const Ctx& c, const void* U, int slot) const = 0;
     virtual void polyakov(const Ctx& c, const void* U, int slot) const = 0;

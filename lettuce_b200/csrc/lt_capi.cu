@@ -1455,9 +1455,7 @@ int lt_clover_timeslices(lt_lattice* h, double* q_t, double* e_t)
     const lt::DeviceScope device_scope(h->device);
     if (!q_t && !e_t) return lt::set_error(LT_ERR_ARG, "lt_clover_timeslices: null pointers");
     const int nt = h->g.n[0];
-    // small lattices spread a timeslice over more blocks (16^4 on two-row links: 84 us with 256 sites a block, 101
-    // with 32)
-    const int per_block = h->g.V >= 65536 ? lt::kRedThreads : 32;
+    const int per_block = h->be->clover_block_sites(h->g);
     const int nbx = std::max(1, std::min(lt::kRedBlocks / nt, (h->g.V / nt + per_block - 1) / per_block));
     if (2 * nt * nbx > lt::kNumSlots * lt::kRedBlocks)
         return lt::set_error(LT_ERR_ARG, "lt_clover_timeslices: more timeslices than the partial-sum buffer holds");

@@ -160,12 +160,16 @@ public:
                                                                       c.partials + (size_t)slot * kRedBlocks);
         finish(c, slot, 1);
     }
-    static constexpr int kCloverSiteMin = 65536;   // two-row links: sites from which one thread takes a site
+    // Two-row links take one thread a site from 16^4 on, the others six warps to 32 sites.  A timeslice is spread
+    // over blocks by the sites that one takes at once: 16^4 FP64 91 us with 32 a block, 95 with 256, 24 x 16^3
+    // 118 and 123; two-row links 16^4 83 us with 256, 101 with 32.
+    static bool clover_by_site(const Geom& g) { return NR == 2 && g.V >= 65536; }
+    int clover_block_sites(const Geom& g) const override { return clover_by_site(g) ? kRedThreads : kSitesPerBlock; }
     void clover_obs(const Ctx& c, const void* U, int slot, bool plaq) const override
     {
         if constexpr (NR == 2)
         {
-            if (!plaq && c.g.V >= kCloverSiteMin)
+            if (!plaq && clover_by_site(c.g))
             {
                 k_clover_site<T, NR><<<kRedBlocks, kRedThreads, 0, c.stream>>>(gauge(U, c.g), c.g,
                                                                                c.partials + (size_t)slot * kRedBlocks);
@@ -246,7 +250,7 @@ public:
     {
         if constexpr (NR == 2)
         {
-            if (c.g.V >= kCloverSiteMin)
+            if (clover_by_site(c.g))
             {
                 k_clover_timeslice<T, NR><<<dim3(nbx, c.g.n[0]), kRedThreads, 0, c.stream>>>(gauge(U, c.g), c.g, partials);
                 return;
