@@ -1,7 +1,10 @@
-"""The Wilson force from the plaquette planes (k_plaq_planes, k_plane_step) in the three storages, as
-a force, as fused kicks and drifts and as flow stages, on lattices with partly empty blocks
-(V = 16, 96, 288, 720 sites against 32 a block) and extents of 2, against the FP64 oracle on the links as
-they are stored.
+"""The Wilson force of all links in the three storages, as a force, as fused kicks and drifts, as the kick that
+ends a trajectory and as flow stages, on lattices with partly empty blocks (V = 16, 96, 288, 720 and 6,000
+sites against 32 a block) and extents of 2, against the FP64 oracle on the links as they are stored.
+
+What runs where: the plaquette planes (k_plaq_planes, k_plane_step) serve FP64 flow stages after the
+first, FP32 ones above 4,736 sites (the last lattice), and FP64 and FP32 kicks after the first drift, the last of
+them without a drift; a force and what comes first take the staple, and two-row links always do.
 
 Bounds: FP64 1e-12.  FP32: a plaquette entry is three products of unit rows, each a sum of three
 complex products rounded by at most 6 eps, the conjugation two more; six of them add up to at most
@@ -16,7 +19,7 @@ from ltref import haar_links_numpy, rel_err
 
 pytestmark = pytest.mark.gpu
 
-EXTS = [(2, 2, 2, 2), (2, 4, 6, 2), (4, 6, 2, 6), (6, 2, 10, 6)]
+EXTS = [(2, 2, 2, 2), (2, 4, 6, 2), (4, 6, 2, 6), (6, 2, 10, 6), (6, 10, 10, 10)]
 TOL = {"fp64": 1e-12, "fp32": 1.1e-5, "fp32_12": 1.1e-5}
 
 
