@@ -202,8 +202,9 @@ public:
         {
             if (split_sweep(c.g))
             {
-                launch_chained(c.g.vh <= 32 * 148 ? k_sweep_split<T, NR, 1, 2> : k_sweep_split<T, NR, 1, 3>, nblocks(c.g.vh, 32), 192, c.stream, gauge(U, c.g), c.g, mu, par,
-                               (T)0, 0, 0u, 0u, 0, c.status, next_order(c));
+                launch_chained(c.g.vh <= 32 * 148 ? k_sweep_split<T, NR, 1, 2> : k_sweep_split<T, NR, 1, 3>,
+                               nblocks(c.g.vh, 32), 192, c.stream, gauge(U, c.g), c.g, mu, par, (T)0, 0, 0u, 0u, 0,
+                               c.status, next_order(c));
                 return;
             }
         }
@@ -224,9 +225,9 @@ public:
         {
             if (split_sweep(c.g))
             {
-                launch_chained(c.g.vh <= 32 * 148 ? k_sweep_split<T, NR, 0, 2> : k_sweep_split<T, NR, 0, 3>, nblocks(c.g.vh, 32), 192, c.stream, gauge(U, c.g), c.g, mu, par,
-                               (T)prefactor, counter, (uint32_t)seed, (uint32_t)(seed >> 32), max_iter, c.status,
-                               next_order(c));
+                launch_chained(c.g.vh <= 32 * 148 ? k_sweep_split<T, NR, 0, 2> : k_sweep_split<T, NR, 0, 3>,
+                               nblocks(c.g.vh, 32), 192, c.stream, gauge(U, c.g), c.g, mu, par, (T)prefactor, counter,
+                               (uint32_t)seed, (uint32_t)(seed >> 32), max_iter, c.status, next_order(c));
                 return;
             }
         }
@@ -576,24 +577,9 @@ public:
     void stout_lambda(const Ctx& c, const void* U, const void* Up, const void* Sigma, void* Lam, void* Lt, void* Tloc,
                       double rho, const void* st_in) const override
     {
-        if (st_in)
-        {
-            launch_chained(k_stout_lambda_st<T, NR>, nblocks(c.g.V, kSitesPerBlock), 4 * kSitesPerBlock, c.stream,
-                           gauge(U, c.g), gauge(Up, c.g), alg(Sigma, c.g), alg(Lam, c.g), alg(Lt, c.g), full(Tloc, c.g),
-                           full(st_in, c.g), c.g, (T)rho);
-            return;
-        }
-        if constexpr (kStaged)
-        {
-            prefer_shared<k_stout_lambda_staged<0>>();
-            launch_chained(k_stout_lambda_staged<0>, nblocks(c.g.V, kSitesPerBlock), 4 * kSitesPerBlock, c.stream,
-                           gauge(U, c.g), gauge(Up, c.g), alg(Sigma, c.g), alg(Lam, c.g), alg(Lt, c.g), full(Tloc, c.g),
-                           c.g, (T)rho);
-            return;
-        }
         launch_chained(k_stout_lambda<T, NR>, nblocks(c.g.V, kSitesPerBlock), 4 * kSitesPerBlock, c.stream,
-                       gauge(U, c.g), gauge(Up, c.g), alg(Sigma, c.g), alg(Lam, c.g), alg(Lt, c.g), full(Tloc, c.g), c.g,
-                       (T)rho);
+                       gauge(U, c.g), gauge(Up, c.g), alg(Sigma, c.g), alg(Lam, c.g), alg(Lt, c.g), full(Tloc, c.g),
+                       full(st_in, c.g), c.g, (T)rho);
     }
     void stout_recursion(const Ctx& c, const void* U, const void* Lam, const void* Lt, const void* Tloc, void* Sigma,
                          double rho) const override

@@ -2157,23 +2157,6 @@ LT_D auto clover_leaves(const F& U, const Geom& g, int par, int i, const int c[4
     return leaf;
 }
 
-// Per-site clover charge density q(x) = ReTr(F01 F23 - F02 F13 + F03 F12), F = C - C^dag
-// (observables/topological_charge.hpp:97-200) and energy density
-// e(x) = sum_{mu<nu} ReTr(F~^2), F~ = Traceless(-i/8 (C - C^dag))
-// (observables/field_strength_tensor.hpp:28-66, :107-134, :154-175).
-// Products run in FP64 for every storage: the cancellations in F = C - C^dag of a smooth
-// (flowed) field would otherwise lift FP32 rounding of the leaves into Q and E.
-//
-// A block is six planes (warps) of 32 sites: each thread multiplies out the four leaves of one plane, takes
-// its share of e, and the planes' H = -i F meet in shared memory, where three warps take the dual pairs of q.
-// One thread a site needed 254 registers for all six planes one after the other and gave an 8^4
-// lattice sixteen blocks.  Bound by the links that come through L2 and, on FP32 storage, by their
-// conversion.  A call for Q and E before and now: FP64 8^4 55 and 33 us, 32 x 24^3 451 and 419; FP32 32^4 963 and
-// 904; two-row FP32 8^4 57 and 33, larger lattices below.  Plaquette, Q and E after a flow step: FP64
-// 8^4 138 and 82 us with the step, two-row FP32 32^4 2319 and 2144.
-//
-// Block (bx, t): timeslice t, or with one row of blocks the whole lattice.  partials: q, e and, with
-// WITH_PLAQ, the plaquette sum, gridDim.y rows of gridDim.x each.
 // The nine reals (herm9_scale) of -i (C - C^dag) of the plane (mu, nu), the leaves of clover_leaves one
 // after the other (the fences keep the loads of the next from being held through this one); plaq: Re tr of the
 // first, the plaquette
@@ -2206,6 +2189,23 @@ LT_D void clover_herm9(const F& U, const Geom& g, int par, int i, const int c[4]
 template <int Unused = 0> LT_D int plane_lo(int pl) { return pl < 3 ? 0 : pl < 5 ? 1 : 2; }
 template <int Unused = 0> LT_D int plane_hi(int pl) { return pl < 3 ? pl + 1 : pl < 5 ? pl - 1 : 3; }
 
+// Per-site clover charge density q(x) = ReTr(F01 F23 - F02 F13 + F03 F12), F = C - C^dag
+// (observables/topological_charge.hpp:97-200) and energy density
+// e(x) = sum_{mu<nu} ReTr(F~^2), F~ = Traceless(-i/8 (C - C^dag))
+// (observables/field_strength_tensor.hpp:28-66, :107-134, :154-175).
+// Products run in FP64 for every storage: the cancellations in F = C - C^dag of a smooth
+// (flowed) field would otherwise lift FP32 rounding of the leaves into Q and E.
+//
+// A block is six planes (warps) of 32 sites: each thread multiplies out the four leaves of one plane, takes
+// its share of e, and the planes' H = -i F meet in shared memory, where three warps take the dual pairs of q.
+// One thread a site needed 254 registers for all six planes one after the other and gave an 8^4
+// lattice sixteen blocks.  Bound by the links that come through L2 and, on FP32 storage, by their
+// conversion.  A call for Q and E before and now: FP64 8^4 55 and 33 us, 32 x 24^3 451 and 419; FP32 32^4 963 and
+// 904; two-row FP32 8^4 57 and 33, larger lattices below.  Plaquette, Q and E after a flow step: FP64
+// 8^4 138 and 82 us with the step, two-row FP32 32^4 2319 and 2144.
+//
+// Block (bx, t): timeslice t, or with one row of blocks the whole lattice.  partials: q, e and, with
+// WITH_PLAQ, the plaquette sum, gridDim.y rows of gridDim.x each.
 template <typename T, int NR, bool WITH_PLAQ>
 __global__ void __launch_bounds__(192, 2) k_clover_obs(Gauge<T, NR> Ust, Geom g, double* __restrict__ partials)
 {
@@ -3129,24 +3129,10 @@ LT_D void stout_lambda_core(const Gauge<T, NR>& Up, const Alg<T>& Sigma, const A
     Tloc.st(mu, par, s, loc);
 }
 
+// The staples St of level k-1 are those that its forward stout step has stored
 template <typename T, int NR>
-__global__ void __launch_bounds__(kThreads, LambdaMinBlocks<T>::value) k_stout_lambda(Gauge<T, NR> U, Gauge<T, NR> Up, Alg<T> Sigma, Alg<T> Lam,
-                                                           Alg<T> Lt, Full<T> Tloc, Geom g, T rho)
-{
-    pdl_release();
-    pdl_wait();
-    int mu, x;
-    if (!link_of_thread(g, mu, x)) return;
-    int par = x >= g.vh, s = x - par * g.vh;
-    int c[4];
-    int i = site_coords(g, par, s, c);
-    stout_lambda_core(Up, Sigma, Lam, Lt, Tloc, rho, mu, par, s, U.ld(mu, par, s), staple(U, g, par, i, c, mu));
-}
-
-// k_stout_lambda with the staple stored by the forward stout step of the level (St)
-template <typename T, int NR>
-__global__ void __launch_bounds__(kThreads, LambdaMinBlocks<T>::value) k_stout_lambda_st(Gauge<T, NR> U, Gauge<T, NR> Up, Alg<T> Sigma, Alg<T> Lam,
-                                                              Alg<T> Lt, Full<T> Tloc, Full<T> St, Geom g, T rho)
+__global__ void __launch_bounds__(kThreads, LambdaMinBlocks<T>::value)
+    k_stout_lambda(Gauge<T, NR> U, Gauge<T, NR> Up, Alg<T> Sigma, Alg<T> Lam, Alg<T> Lt, Full<T> Tloc, Full<T> St, Geom g, T rho)
 {
     pdl_release();
     pdl_wait();
@@ -3154,25 +3140,6 @@ __global__ void __launch_bounds__(kThreads, LambdaMinBlocks<T>::value) k_stout_l
     if (!link_of_thread(g, mu, x)) return;
     const int par = x >= g.vh, s = x - par * g.vh;
     stout_lambda_core(Up, Sigma, Lam, Lt, Tloc, rho, mu, par, s, U.ld(mu, par, s), St.ld(mu, par, s));
-}
-
-// k_stout_lambda on two-row FP32 storage with the staged staple
-template <int Unused = 0>
-__global__ void __launch_bounds__(4 * kSitesPerBlock, LT_MINB_LAMBDA_F32)
-    k_stout_lambda_staged(Gauge<float, 2> U, Gauge<float, 2> Up, Alg<float> Sigma, Alg<float> Lam, Alg<float> Lt,
-                          Full<float> Tloc, Geom g, float rho)
-{
-    __shared__ StapleRing ring;
-    pdl_release();
-    pdl_wait();
-    int mu, x;
-    if (!link_of_thread(g, mu, x)) return;
-    const int par = x >= g.vh, s = x - par * g.vh;
-    int c[4];
-    const int i = site_coords(g, par, s, c);
-    M3<float> u;
-    const M3<float> st = staple_staged<true>(ring, U, g, par, i, s, c, mu, u);
-    stout_lambda_core(Up, Sigma, Lam, Lt, Tloc, rho, mu, par, s, u, st);
 }
 
 // Second half of StoutForceRecursion (smearing/stout_smearing.hpp:177-230):
