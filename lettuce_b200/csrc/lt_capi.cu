@@ -54,7 +54,15 @@ struct DevStore
         if (limit && bytes + n > limit) return cudaErrorMemoryAllocation;
         const cudaError_t e = cudaMalloc(p, n);
         if (e != cudaSuccess) return e;
-        size[*p] = n;
+        try
+        {
+            size[*p] = n;
+        }
+        catch (...)
+        {
+            cudaFree(*p);
+            return cudaErrorMemoryAllocation;
+        }
         bytes += n;
         return e;
     }
@@ -170,7 +178,14 @@ void dev_lend(int device, void** p, cudaStream_t stream, bool keep)
 {
     std::lock_guard<std::mutex> lk(g_store_mutex);
     DevStore& st = stores()[device];
-    if (!keep) st.idle[p] = stream;
+    try
+    {
+        if (!keep) st.idle[p] = stream;
+    }
+    catch (...)
+    {
+        // no host memory for the entry: the buffer stays with its handle
+    }
     --st.borrowed;
     --t_borrowed;
     st.returned.notify_all();
@@ -203,8 +218,15 @@ void dev_free(int device, void** p)
     else
     {
         if (st.kept_bytes + bytes > st.most) st.give_back(bytes);
-        st.kept.emplace_back(bytes, *p);
-        st.kept_bytes += bytes;
+        try
+        {
+            st.kept.emplace_back(bytes, *p);
+            st.kept_bytes += bytes;
+        }
+        catch (...)
+        {
+            st.drop(*p);
+        }
     }
     *p = nullptr;
 }
