@@ -26,7 +26,9 @@ struct Ctx
     // forces over all links; null: no memory for them, the rectangles are multiplied out directly
     void* rectD = nullptr;
     void* rectE = nullptr;
-    void* planes = nullptr;       // plaquette planes of the Wilson force (plane_bytes); null: no memory for them
+    // plaquette planes of the Wilson force (plane_bytes); null: no memory for them, or links as given, which
+    // need not be unitary
+    void* planes = nullptr;
     unsigned* order = nullptr;    // the handle's launch counter for alternating site orders
 };
 
@@ -92,8 +94,8 @@ public:
                         uint64_t seed, int max_iter) const = 0;
     virtual void heatbath(const Ctx& c, void* U, int mu, int par, double prefactor, uint64_t counter,
                           uint64_t seed, int max_iter) const = 0;
-    // flow_split(): the format runs a flow stage without planes as two kernels and wants an algebra
-    // scratch field X (flow_stage's last argument; null: the fused stage)
+    // flow_split(): the format runs a flow stage without planes as two kernels and needs an algebra
+    // field X (flow_stage's last argument)
     virtual bool flow_split() const = 0;
     virtual void flow_stage(const Ctx& c, const void* Uin, void* Uout, void* Z, double c_old, double c_new,
                             double c_exp, int read_z, int write_z, void* X) const = 0;

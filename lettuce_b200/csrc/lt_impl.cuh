@@ -322,18 +322,20 @@ public:
             plane_step<Step::Flow>(c, Uin, Uout, Z, nullptr, c_old, c_new, c_exp, read_z, write_z);
             return;
         }
+        const int nb = nblocks(c.g.V, kSitesPerBlock);
         if constexpr (std::is_same<T, double>::value)
         {
-            if (X)
-            {
-                const int nb = nblocks(c.g.V, kSitesPerBlock);
-                force(c, Uin, X, c.rect, c.cp, c.cr);
-                launch_chained(k_flow_update<T, NR>, nb, 4 * kSitesPerBlock, c.stream, gauge(Uin, c.g),
-                               gauge(Uout, c.g), alg(Z, c.g), alg(X, c.g), c.g, (T)c_old, (T)c_new, (T)c_exp, read_z,
-                               write_z, next_order(c));
-                return;
-            }
+            force(c, Uin, X, c.rect, c.cp, c.cr);
+            launch_chained(k_flow_update<T, NR>, nb, 4 * kSitesPerBlock, c.stream, gauge(Uin, c.g), gauge(Uout, c.g),
+                           alg(Z, c.g), alg(X, c.g), c.g, (T)c_old, (T)c_new, (T)c_exp, read_z, write_z, next_order(c));
         }
+        else
+            flow_stage_fused(c, Uin, Uout, Z, c_old, c_new, c_exp, read_z, write_z);
+    }
+    // The stage in one kernel, FP32 links
+    static void flow_stage_fused(const Ctx& c, const void* Uin, void* Uout, void* Z, double c_old, double c_new,
+                                 double c_exp, int read_z, int write_z)
+    {
         const int nb = nblocks(c.g.V, kSitesPerBlock);
         const Act a = act(c, c.rect);
         if (a == Act::TwoLink) prepare_rect(c, Uin, c.cr);

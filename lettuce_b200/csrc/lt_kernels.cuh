@@ -1846,9 +1846,10 @@ __global__ void __launch_bounds__(4 * kSitesPerBlock, LT_MINB_FLOW_STAGED)
 // F_{mu nu}(x) = Algebra(P_{mu nu}(x)), P the plaquette that starts at x along mu,
 //   Algebra(st U_mu(x)^dag) = sum_{nu != mu} [U_nu(x-nu)^dag F_{mu nu}(x-nu) U_nu(x-nu) - F_{mu nu}(x)]:
 // the upper staples close to P_{nu mu}(x) = P_{mu nu}(x)^dag, the lower ones to the plaquette at x - nu
-// carried along the link between them.  Every plaquette is multiplied out once for its four links
-// instead of once for each: 870 multiply-adds a link for the force against 1,390 from the staple, and
-// 8 link loads against 19, at far fewer registers (FP64: 140 and 160 in the two kernels, 255 in the
+// carried along the link between them, which holds for unitary links: the first stage of a flow and the kicks
+// before the first drift, on links as given, take the staple.  Every plaquette is multiplied out once for its
+// four links instead of once for each: 870 multiply-adds a link for the force against 1,390 from the staple,
+// and 8 link loads against 19, at far fewer registers (FP64: 132 and 160 in the two kernels, 255 in the
 // staple's).  Bound by issue and HBM together (the planes cross it once each way).  An RK3 stage, before and
 // now: FP64 32^4 1129 and 923 us, 16^4 65 and 51; FP32 32^4 611 and 491, 16^4 33 and 27; a kick and its
 // drift FP64 32^4 1050 and 941, FP32 606 and 501.  Working through slabs of timeslices, so that the planes
@@ -2006,9 +2007,9 @@ __global__ void __launch_bounds__(4 * kSitesPerBlock, LT_MINB_STAGED)
 }
 
 // The second half of a split flow stage: Z <- c_old Z + c_new X, U' = exp(c_exp Z) U, with
-// X = Algebra(st U^dag) from k_flow_force.  FP64 links run a rectangle stage (and, where there is no
-// memory for the plaquette planes, a Wilson stage) as these two kernels: the fused stage needs 254
-// registers (two blocks of 128 per SM), the halves far fewer each.
+// X = Algebra(st U^dag) from k_flow_force.  FP64 links run a rectangle stage (and a Wilson stage without
+// plaquette planes: the first of a flow, or where there is no memory for them) as these two kernels: the fused
+// stage needs 254 registers (two blocks of 128 per SM), the halves far fewer each.
 template <typename T, int NR>
 __global__ void __launch_bounds__(kThreads) k_flow_update(Gauge<T, NR> Uin, Gauge<T, NR> Uout, Alg<T> Z, Alg<T> X,
                                                           Geom g, T c_old, T c_new, T c_exp, int read_z, int write_z,
@@ -2959,7 +2960,8 @@ template <typename T> struct CloverCornersMinBlocks
 // V^dag (W^dag K(x-nu) + K(x+mu-nu) W^dag) U_nu(x-nu) under it: 8 products instead of 16 for every link and
 // nu, for one conjugation per (nu, mu, site) done once.  Bound by instruction issue like the direct form.  The
 // whole force of four stout levels, with Lt in the recursion below, before and now: two-row FP32 16^4
-// 551 and 501 us, 24^4 2580 and 2382; FP32 574 and 535; FP64 1148 and 1111 (corners only).
+// 541 and 508 us, 24^4 2586 and 2402; FP32 574 and 540; FP64 1154 and 1119 (corners only).  Takes the links for
+// unitary, as every smeared level is.
 template <typename T> LT_HD int k_plane(int nu, int mu) { return 3 * nu + mu - (mu > nu ? 1 : 0); }
 
 template <typename T, int NR>
@@ -3146,7 +3148,8 @@ __global__ void __launch_bounds__(kThreads, LambdaMinBlocks<T>::value)
 // Sigma_{k-1} = Algebra(U (Tloc - i rho sum_{nu != mu} [six-term neighbour sum of U and Lambda]))
 // With Lt = U^dag Lambda U of every link (written beside Lambda) the terms over the link are
 //   U_nu(x+mu) [U_mu(x+nu)^dag (Lambda_mu(x+nu) + Lt_nu(x)) - Lt_nu(x+mu) U_mu(x+nu)^dag] U_nu(x)^dag,
-// four products instead of six, as many as those under it; without Lt (no memory for it) the six.
+// four products instead of six, as many as those under it; without Lt (no memory for it, or links as given, which
+// need not be unitary) the six.
 template <typename T> struct RecursionMinBlocks
 {
     static constexpr int value = sizeof(T) == 4 ? 4 : 1;
